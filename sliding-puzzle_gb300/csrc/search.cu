@@ -8,23 +8,28 @@
 //
 //  * one lane = one depth-first search over a task (a root-set node, possibly
 //    narrowed to some of its first moves); no block barriers in the loop;
-//  * the lane's path kept as 2-bit moves in shared memory (a [word][lane]
-//    layout, so lanes never conflict on banks) and undone move by move;
-//  * 15-puzzle boards packed 4 bits per cell in one 64-bit register, 24-puzzle
-//    boards as bytes in shared memory;
-//  * Manhattan distance updated from a per-(move, cell, tile) delta table in
-//    shared memory (src/15puzzle_block_parallel.cu:271-272 updates it with two
-//    constant-memory lookups);
+//  * the lane's whole state that is indexed by cell, pattern or level in
+//    shared memory, one column of words per lane (LaneRows below), so that no
+//    index costs a bank conflict, a 64-bit shift or a select;
+//  * what a move changes from one table entry per (tile, cell, move): the
+//    pattern-index changes or the Manhattan change
+//    (src/15puzzle_block_parallel.cu:271-272 takes two constant-memory
+//    lookups), and the child's move mask;
 //  * PDB indices kept per pattern as mixed-radix integers and updated by one
 //    add per move, so a generated child costs one regular and one reflected
 //    table lookup instead of the reference's eight
 //    (src/24puzzle_block_parallel_with_pdb.cu:426-429); the idea of updating
 //    only the moved tile's pattern is Horie's (src_horie/idas_pdb.cu:221-254);
-//    undoing a move restores the two overwritten pattern values from a
-//    per-level save in shared memory instead of looking them up again;
+//    undoing a move restores the two overwritten values from the level's
+//    bytes instead of looking them up again;
 //  * generating a child and undoing a move share one code path (both slide
-//    one tile into the blank), which keeps a warp's lanes converged while
-//    they are at different points of their walks;
+//    one tile into the blank), and the warp's lanes are held together on it.
+//    Bound by issue and by table reads in flight.  Against the version with
+//    register boards and indices, whose lanes drifted apart (9-15 of 32
+//    active per instruction, 18-21 warp instructions per node; now 18 and
+//    10): 100 random 15-puzzles 28.8 -> 19.7 ms, 4096 mixed ones 348 -> 211
+//    ms (70 -> 116 G nodes/s), 100 Manhattan walks 29.2 -> 18.9 ms, 16384
+//    24-puzzle roots 166 -> 101 ms;
 //  * load balance by a device task pool: lanes claim slots warp-aggregated
 //    (ballot + one atomicAdd per warp); claims may run ahead of the pool's
 //    tail, and while any lane waits, busy lanes donate the untried moves of
@@ -85,41 +90,24 @@ __device__ __forceinline__ unsigned long long globaltimer() {
   return t;
 }
 
-// Pattern-index field helpers.  Width 4: three 20-bit indices in one u64 per
-// partition.  Width 5: four 28-bit indices, two per u64.
+// Field p of packed pattern indices (HeurTables::sum): width 4 three 20-bit
+// fields in one word, width 5 four 28-bit fields, two to a word.
 template <int W>
-struct Idx;
+__device__ __forceinline__ uint32_t sum_field(uint64_t a, uint64_t b, int p) {
+  if (W == 4) return (uint32_t)(a >> (20 * p)) & 0xFFFFFu;
+  return (uint32_t)((p >> 1 ? b : a) >> (28 * (p & 1))) & 0xFFFFFFFu;
+}
 
-template <>
-struct Idx<4> {
-  uint64_t a;
-  __device__ __forceinline__ void clear() { a = 0; }
-  __device__ __forceinline__ uint32_t get(int p) const { return (uint32_t)(a >> (20 * p)) & 0xFFFFFu; }
-  __device__ __forceinline__ void add(int p, int32_t d) { a += (uint64_t)((int64_t)d << (20 * p)); }
-};
-
-template <>
-struct Idx<5> {
-  uint64_t a, b;
-  __device__ __forceinline__ void clear() { a = b = 0; }
-  __device__ __forceinline__ uint32_t get(int p) const {
-    uint64_t w = (p >> 1) ? b : a;
-    return (uint32_t)(w >> (28 * (p & 1))) & 0xFFFFFFFu;
-  }
-  __device__ __forceinline__ void add(int p, int32_t d) {
-    uint64_t v = (uint64_t)((int64_t)d << (28 * (p & 1)));
-    if (p >> 1) b += v; else a += v;
-  }
-};
-
-__device__ __forceinline__ uint32_t byte_sum(uint32_t v) { return __dp4a(v, 0x01010101u, 0u); }
-
-// The step's move arithmetic without compares: the four blank
-// displacements as signed bytes of one immediate, and for the 24-puzzle the
-// 4-bit legal-move mask of every cell packed into two 64-bit immediates
-// (measured: -3 % step time on the 15-puzzle for the first, +5 % nodes/s on
-// the 24-puzzle for both; the packed masks cost the 15-puzzle kernel a
-// spill, so it keeps legal_moves).
+// Blank displacement of move d without compares: the four displacements as
+// signed bytes of one immediate, byte d sign-extended by one permute.
+template <int W>
+__device__ __forceinline__ int step_delta(uint32_t d) {
+  constexpr uint32_t pack = W == 4 ? 0x04FF01FCu : 0x05FF01FBu;  // -W, +1, -1, +W
+  int r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(pack), "r"(d * 0x1111u + 0x8880u));
+  return r;
+}
+// legal_moves from 4-bit masks of every cell packed into 64-bit immediates.
 constexpr uint64_t legal_pack(int w, int first, int count) {
   uint64_t v = 0;
   for (int c = 0; c < count; ++c) {
@@ -131,18 +119,12 @@ constexpr uint64_t legal_pack(int w, int first, int count) {
 }
 template <int W>
 __device__ __forceinline__ uint32_t step_legal(int blank) {
-  if (W == 4) return legal_moves(W, blank);
-  const uint64_t w = blank < 16 ? legal_pack(5, 0, 16) : legal_pack(5, 16, 9);
+  const uint64_t w = W == 4 ? legal_pack(4, 0, 16) : blank < 16 ? legal_pack(5, 0, 16) : legal_pack(5, 16, 9);
   return (uint32_t)(w >> (4 * (blank & 15))) & 15u;
 }
-template <int W>
-__device__ __forceinline__ int step_delta(int d) {
-  constexpr uint32_t pack = W == 4 ? 0x04FF01FCu : 0x05FF01FBu;  // -W, +1, -1, +W
-  return (int)(pack << (24 - 8 * d)) >> 24;
-}
-__device__ __forceinline__ uint32_t set_byte(uint32_t v, int p, uint32_t x) {
-  return (v & ~(0xFFu << (8 * p))) | (x << (8 * p));
-}
+// Lowest move of a non-empty 4-bit move mask: sixteen 2-bit answers in one
+// immediate.
+__device__ __forceinline__ uint32_t first_move(uint32_t mask) { return (0x12131210u >> (2 * mask)) & 3u; }
 
 }  // namespace
 
@@ -388,9 +370,6 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
   }
 }
 
-// Resident threads per SM the search kernels are compiled for (the register
-// budget: 768 threads leave 80 registers a thread; 24 warps per SM hide the
-// pattern-table latency markedly better than 16).
 // Most lanes of a warp that donate in one pass of its loop.
 #ifndef SP_MAX_DONORS
 #define SP_MAX_DONORS 8
@@ -401,33 +380,95 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
 #define SP_MAX_BACKOFF_NS 16384
 #endif
 
-#ifndef SP_SEARCH_THREADS_PER_SM
-#define SP_SEARCH_THREADS_PER_SM 768
-#endif
+// Resident threads per SM that the search kernels are compiled for, and the
+// shared memory that these may take together.  The PDB search is bound by its
+// table reads in flight: a read that misses L1 holds an L1 line until L2
+// answers, so the part of the SM's 256 KB that is left to L1 limits them.  At
+// 228 KB of shared memory (28 KB of L1) a batch of 4096 15-puzzles took 288
+// ms and a 16384-root round of the 24-puzzle 148 ms, at up to 196 KB 247 and
+// 102 ms, and only with the larger L1 do more warps pay: 1024 threads (64
+// registers, nothing spilled) 220 ms.  The 24-puzzle's rows are longer: at
+// 1024 threads its shared levels would shrink from 48 to 28 (100 against 102
+// ms, but a batch of 50 12.1 against 11.5 ms).  Manhattan reads no tables:
+// 768 or 1024 threads measure alike.
+constexpr int kSharedPerSm = 192 * 1024;
+constexpr int threads_per_sm(int w, bool pdb) { return pdb && w == 4 ? 1024 : 768; }
+
+// What a lane keeps in shared memory: 32-bit words, one column per lane
+// ([row][thread]), so that a lane only ever touches its own bank whatever
+// cell, pattern or level it indexes (a byte of a word included).
+//   board   4 cells to a word, a byte each; the blank's own byte is stale
+//   index   PDB: per pattern its table index with the table's base in it
+//           (width 4: base in bits 20-21 and the table value in bits 24-31;
+//           width 5: base in bit 28, the values as bytes of two more words)
+//   cold    data of rare events
+//   level   per level of the walk a byte with the moves still untried there
+//           (bits 0-3) and the reverse of the move taken (bits 4-5) and, for
+//           the PDB, a byte in each of two more planes: the regular and the
+//           reflected table value that move overwrote; PDB levels beyond the
+//           shared ones are in local memory
+// The level bytes hold what an undo needs, so it neither recomputes the
+// move mask nor reads a table, and donating a level is clearing its mask.
+template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
+struct LaneRows {
+  static constexpr int N = W * W;
+  static constexpr int kMaxLev = WORDS * 16;
+  static constexpr int kPat = W == 4 ? 3 : 4;
+  static constexpr int kBoard = 0;
+  static constexpr int kIdx = kBoard + (N + 3) / 4;
+  static constexpr int kVal = kIdx + (PDB ? 2 * kPat : 0);
+  static constexpr int kCold = kVal + (PDB && W == 5 ? 2 : 0);
+  static constexpr int kLevel = kCold + 6;
+  // move tables of the block (bytes), pool cache and publication buckets
+  static constexpr int kMoveTable = PDB ? (W == 4 ? 8 * 4 * N * N : 8 * N * N + 4 * N) : 4 * N * N;
+  static constexpr int kFixed = kMoveTable + 64 + (MULTI ? BLOCK * 4 : 4) + BLOCK / 32 * 64;
+  // shared levels: what fits beside the rest (1 KB is reserved per block)
+  static constexpr int kBudget = kSharedPerSm / (threads_per_sm(W, PDB) / BLOCK) - 1024;
+  static constexpr int kFit = (kBudget - kFixed) / (4 * BLOCK) - kLevel;
+  static constexpr int kShared = PDB && kFit / 3 * 4 < kMaxLev ? kFit / 3 * 4 : kMaxLev;
+  static constexpr int kDeep = kMaxLev - kShared;
+  static constexpr int kPlane = kShared / 4;  // rows of one plane of level bytes
+  static constexpr int kRows = kLevel + (PDB ? 3 : 1) * kPlane;
+};
+
+// What a warp keeps in shared memory: its statistics and, for its idle spells,
+// the pool state it last saw.
+struct WarpState {
+  unsigned long long steps, slots, idle, begin, last_change;
+  uint32_t last_out, last_tail, last_hb, beat, backoff, pad;
+};
+static_assert(sizeof(WarpState) == 64, "WarpState layout");
 
 template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
-__global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) search_round_kernel(RoundParams P) {
+__global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_round_kernel(RoundParams P) {
+  using R = LaneRows<W, PDB, BLOCK, WORDS, MULTI>;
   constexpr int N = W * W;
-  constexpr int BSTRIDE = 28;  // bytes per lane board (7 words: conflict-free same-cell access)
-  constexpr int MAXLEV = WORDS * 16;
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ uint32_t s_code[PDB ? 2 * N * N : 1];
-  __shared__ uint8_t s_pat[PDB ? 2 * N : 1];
-  __shared__ int8_t s_mdd[PDB ? 1 : 4 * N * N];
-  __shared__ uint32_t s_stack[WORDS][BLOCK];
-  __shared__ uint32_t s_prefix[kPathWords][BLOCK];  // the lane's task prefix (its pool slot is freed)
-  // PDB: the two pattern values (regular, reflected) a descent overwrote, per
-  // level, so that backtracking restores them without table lookups; levels
-  // from HSAVE on look them up again
-  constexpr int HSAVE = PDB ? (W == 4 ? 64 : 32) : 1;
-  __shared__ uint16_t s_hsave[HSAVE][BLOCK];
-  __shared__ __align__(16) uint8_t s_board[W == 5 ? BLOCK * BSTRIDE : 4];
+  // One entry per (tile, cell it slides from, blank's move): what the step
+  // needs of a move in one shared read.
+  //   PDB, width 4: per partition the pattern-index change << 8 | pattern; the
+  //     regular one also holds the child's move mask (legal, not the reverse)
+  //     in bits 4-7
+  //   PDB, width 5: the change is the difference of two (tile, cell) codes
+  //     (a full table would take 20 KB), the pattern in their top 4 bits
+  //   Manhattan: the child's move mask, bit 4 set when the tile gets farther
+  __shared__ uint2 s_mv[PDB ? (W == 4 ? 4 * N * N : N * N) : 1];
+  __shared__ uint8_t s_rem[PDB && W == 5 ? 4 * N : 4];
+  __shared__ uint8_t s_md[PDB ? 4 : 4 * N * N];
+  __shared__ uint32_t s_lane[R::kRows][BLOCK];
   // multi-iteration mode: per-warp bucket counts of the longest-first publication
   __shared__ uint32_t s_hist[MULTI ? BLOCK / 32 : 1][32];
-  __shared__ uint32_t s_cold[3][BLOCK];  // per-lane data of rare events (below)
   // block-wide cache of the pool state: at most one global poll per block per poll_ns
   __shared__ uint32_t s_pool[5];  // head, tail, error, outstanding, heartbeat
   __shared__ unsigned long long s_pool_t;
+  __shared__ WarpState s_warp[BLOCK / 32];
+  __shared__ uint32_t s_stat[5];  // donation counters: tries, slot not free, hungry polls, tasks done, donor found
+  if (threadIdx.x < 5) s_stat[threadIdx.x] = 0;
+  if ((threadIdx.x & 31) == 0) {
+    s_warp[threadIdx.x >> 5] = WarpState{};
+    s_warp[threadIdx.x >> 5].begin = (unsigned long long)clock64();
+    s_warp[threadIdx.x >> 5].backoff = 256;
+  }
   if (threadIdx.x == 0) {
     s_pool[0] = s_pool[1] = s_pool[2] = s_pool[4] = 0;
     s_pool[3] = 1;
@@ -436,115 +477,163 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
   }
 
   const HeurTables *ht = P.ht;
-  if (PDB) {
+  auto child_moves = [](int cell, int d) -> uint32_t { return legal_moves(W, cell) & ~(1u << (3 - d)); };
+  if (PDB && W == 5) {
     for (int i = threadIdx.x; i < N * N; i += BLOCK) {
-      s_code[i] = ht->code[0][i];
-      s_code[N * N + i] = ht->code[1][i];
+      const int t = i / N;
+      s_mv[i] = make_uint2(ht->code[0][i] | (uint32_t)ht->pat[0][t] << 28,
+                           ht->code[1][i] | (uint32_t)ht->pat[1][t] << 28);
     }
-    for (int i = threadIdx.x; i < N; i += BLOCK) {
-      s_pat[i] = ht->pat[0][i];
-      s_pat[N + i] = ht->pat[1][i];
-    }
+    for (int i = threadIdx.x; i < 4 * N; i += BLOCK) s_rem[i] = (uint8_t)child_moves(i / 4, i % 4);
   } else {
-    for (int i = threadIdx.x; i < 4 * N * N; i += BLOCK) s_mdd[i] = ht->mdd[i];
+    for (int i = threadIdx.x; i < 4 * N * N; i += BLOCK) {
+      const int d = i % 4, c = (i / 4) % N, t = i / (4 * N);
+      const int to = c - move_delta(W, d);
+      const bool legal = to >= 0 && to < N && ((legal_moves(W, to) >> d) & 1u);
+      if (PDB) {
+        uint2 v = make_uint2(0, 0);
+        if (legal && t) {
+          v.x = (ht->code[0][t * N + to] - ht->code[0][t * N + c]) << 8 | child_moves(c, d) << 4 | ht->pat[0][t];
+          v.y = (ht->code[1][t * N + to] - ht->code[1][t * N + c]) << 8 | ht->pat[1][t];
+        }
+        s_mv[i] = v;
+      } else {
+        s_md[i] = (uint8_t)(child_moves(c, d) | (legal && ht->mdd[(d * N + c) * N + t] > 0 ? 16u : 0u));
+      }
+    }
   }
   __syncthreads();
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  uint8_t *myboard = s_board + (W == 5 ? tid * BSTRIDE : 0);
+  uint32_t *const me = &s_lane[0][tid];                      // row r of the lane: me[r * BLOCK]
+  uint8_t *const mb = reinterpret_cast<uint8_t *>(me);
+  // local memory: the task's moves above its start (its pool slot is freed),
+  // and the levels beyond the shared ones, their three bytes in a word
+  uint32_t prefix[kPathWords], deep[R::kDeep > 0 ? R::kDeep : 1];
+  WarpState &ws = s_warp[tid >> 5];
+  uint32_t *const s_cold0 = s_lane[R::kCold], *const s_cold1 = s_lane[R::kCold + 1],
+           *const s_cold2 = s_lane[R::kCold + 2];
+  // the task's SubRoot; its instance (multi-iteration mode: bit 31 = the
+  // parity of the task's iteration); its split levels (a split task hands
+  // every node at relative depth 1 to the pool)
+  uint32_t &sub = s_lane[R::kCold + 3][tid], &cur_inst = s_lane[R::kCold + 4][tid],
+           &splitk = s_lane[R::kCold + 5][tid];
   PoolCtl *ctl = P.ctl;
 
   // ---- lane state -------------------------------------------------------
   int state = 0;  // 0 idle, 1 holds a claimed slot, 2 searching
   uint32_t slot = 0;
-  uint64_t b64 = 0;  // width-4 board
-  int blank = 0, g = 0, h = 0, k = 0, it = 0, pre = -1, limit = 0;
-  int rblank = 0, rpre = -1, groot = 0, plen = 0;
-  uint32_t mask0 = 0, top = 0, sub = 0;
-  uint64_t cut = 0;
-  uint32_t lo = 0;  // donation walk cache: level | blank << 8 | (incoming move + 1) << 16
-  unsigned long long cnt = 0;
-  Idx<W> ir, iff;
-  uint32_t hvr = 0, hvf = 0;
-  ir.clear();
-  iff.clear();
-  unsigned long long c_tries = 0, c_notfree = 0, c_nowait = 0, c_done = 0, c_found = 0;  // donation counters
-  // the task's instance; multi-iteration mode: bit 31 = the parity of the
-  // task's iteration (kept in the same register: the search loop has none to spare)
-  uint32_t cur_inst = 0;
-  int splitk = 0;         // split task: hand every node at this relative depth to the pool
-  bool emit_pending = false;
+  int blank = 0, k = 0;
+  uint32_t boff = 0;             // board_off(blank)
+  uint32_t rem = 0;              // moves still untried at the current node
+  int hr = 0, hf = 0;            // h of the two partitions (Manhattan: hr alone)
+  int budget = 0;                // a child of level k is entered when its h <= budget - k
+  int kstop = 0;                 // entering a child of this level is special: the first of a split
+                                 // task, else the last that the lane's stack and path can hold
+  int groot = 0, plen = 0;
+  int lo = 0;                    // donation: no level below lo has untried moves
+  uint32_t cnt = 0;              // generated nodes not yet added to the task's counters
   // Rare per-lane events, flags in a register and their data in shared memory:
   //  * kAdvance: the lane finished an instance's iteration; the warp advances
-  //    that instance (s_cold[0]) at the top of its next loop;
-  //  * kDebt: a reserved pool index (s_cold[1]) whose ring slot did not free
+  //    that instance (s_cold0) at the top of its next loop;
+  //  * kDebt: a reserved pool index (s_cold1) whose ring slot did not free
   //    in time is owed: the lane kept the work and publishes a null task (no
-  //    moves, SubRoot s_cold[2]) there later, so no index stays unpublished.
+  //    moves, SubRoot s_cold2) there later, so no index stays unpublished.
   constexpr uint32_t kAdvance = 1u, kDebt = 2u;
   uint32_t events = 0;
 
-  auto tile_at = [&](int c) -> int {
-    if (W == 4) return (int)((b64 >> (4 * c)) & 15u);
-    return myboard[c];
+  auto board_off = [&](int c) -> uint32_t {
+    return (uint32_t)c + (uint32_t)(c >> 2) * (4u * BLOCK - 4u) + 4u * BLOCK * R::kBoard;
   };
-  // slide tile t from cell `from` into the blank at cell `to`
-  auto slide = [&](int t, int from, int to) {
-    if (W == 4) {
-      b64 ^= ((uint64_t)t << (4 * from)) ^ ((uint64_t)t << (4 * to));
-    } else {
-      myboard[to] = (uint8_t)t;
-      myboard[from] = 0;
+  auto level_off = [&](int j) -> uint32_t {
+    return (uint32_t)j + (uint32_t)(j >> 2) * (4u * BLOCK - 4u) + 4u * BLOCK * R::kLevel;
+  };
+  auto level_get = [&](int j) -> uint32_t {
+    return R::kDeep > 0 && j >= R::kShared ? deep[j - R::kShared] & 0xFFu : mb[level_off(j)];
+  };
+  auto level_cut = [&](int j) {  // no move of level j is left to try
+    if (R::kDeep > 0 && j >= R::kShared) deep[j - R::kShared] &= ~15u;
+    else mb[level_off(j)] &= (uint8_t)~15u;
+  };
+  // The lane's first `len` moves below its SubRoot -- the task's prefix, then
+  // its walk's first len - plen levels -- as words handed to put(index, word).
+  // The levels come four to a shared word: the complement of bits 4-5 of
+  // each byte, squeezed to 8 bits.
+  auto write_path = [&](int len, auto put) {
+    int wi = 0;
+    for (; 16 * (wi + 1) <= plen; ++wi) put(wi, prefix[wi]);
+    const int lev = len - plen;
+    uint32_t acc = 0;
+    int at = plen & 15;  // moves in acc
+    if (at) acc = prefix[wi] & ((1u << (2 * at)) - 1u);
+    for (int j = 0; j < lev; j += 4) {
+      uint32_t x = 0;
+      if (R::kDeep > 0 && j >= R::kShared) {
+        for (int q = j; q < min(j + 4, R::kMaxLev); ++q) x |= (deep[q - R::kShared] & 0xFFu) << (8 * (q - j));
+      } else {
+        x = me[(R::kLevel + (j >> 2)) * BLOCK];
+      }
+      x = ~(x >> 4) & 0x03030303u;
+      x = (x | x >> 6 | x >> 12 | x >> 18) & 0xFFu;
+      const int n = min(4, lev - j);
+      if (n < 4) x &= (1u << (2 * n)) - 1u;
+      acc |= x << (2 * at);
+      at += n;
+      if (at >= 16) {
+        put(wi++, acc);
+        at -= 16;
+        acc = at ? x >> (2 * (n - at)) : 0u;
+      }
     }
+    if (at) put(wi, acc);
   };
-  auto lookup = [&](int p, uint32_t idx) -> uint32_t {
-    size_t off = (W == 4) ? ((size_t)p << 20) : (p ? ((size_t)1 << 28) : 0);
-    return __ldg(P.pdb + off + idx);
-  };
-  auto stack_dir = [&](int i) -> int {
-    uint32_t w = ((i >> 4) < (k >> 4)) ? s_stack[i >> 4][tid] : top;
-    return (int)((w >> (2 * (i & 15))) & 3u);
-  };
-  auto task_dir = [&](int i) -> int {
-    return (int)((s_prefix[i >> 4][tid] >> (2 * (i & 15))) & 3u);
-  };
-  // moves 0..len-1 of the lane's path below its SubRoot: task prefix then stack
-  auto path_word = [&](int wi, int len) -> uint32_t {
-    uint32_t out = 0;
-    for (int b = 0; b < 16; ++b) {
-      int j = wi * 16 + b;
-      if (j >= len) break;
-      int d = j < plen ? task_dir(j) : stack_dir(j - plen);
-      out |= (uint32_t)d << (2 * b);
-    }
-    return out;
-  };
+  auto lookup = [&](uint32_t off) -> uint32_t { return __ldcg(P.pdb + off); };
+  // h of the lane's board (its blank byte 0) from nothing: pattern indices
+  // and table values too
   auto full_h = [&]() -> int {
     if (PDB) {
-      ir.clear();
-      iff.clear();
+      uint64_t ra = 0, rb = 0, fa = 0, fb = 0;
+#pragma unroll 4
       for (int c = 0; c < N; ++c) {
-        int t = tile_at(c);
-        if (!t) continue;
-        ir.add(s_pat[t], (int32_t)s_code[t * N + c]);
-        iff.add(s_pat[N + t], (int32_t)s_code[N * N + t * N + c]);
+        const uint32_t t = mb[4 * BLOCK * (R::kBoard + c / 4) + c % 4];
+        const ulonglong2 *rec = reinterpret_cast<const ulonglong2 *>(ht->sum) + (t * N + c) * (W == 4 ? 1u : 2u);
+        const ulonglong2 v = __ldg(rec);
+        if (W == 4) {
+          ra += v.x;
+          fa += v.y;
+        } else {
+          const ulonglong2 u = __ldg(rec + 1);
+          ra += v.x;
+          rb += v.y;
+          fa += u.x;
+          fb += u.y;
+        }
       }
-      hvr = hvf = 0;
-      constexpr int NP = (W == 5) ? 4 : 3;
-      for (int p = 0; p < NP; ++p) {
-        hvr = set_byte(hvr, p, lookup(W == 5 ? (p != 0) : p, ir.get(p)));
-        hvf = set_byte(hvf, p, lookup(W == 5 ? (p != 0) : p, iff.get(p)));
+      hr = hf = 0;
+#pragma unroll
+      for (int p = 0; p < R::kPat; ++p) {
+        const uint32_t base = W == 4 ? (uint32_t)p << 20 : (p ? 1u << 28 : 0u);
+        const uint32_t a = sum_field<W>(ra, rb, p) | base, b = sum_field<W>(fa, fb, p) | base;
+        const uint32_t va = lookup(a), vb = lookup(b);
+        me[(R::kIdx + p) * BLOCK] = W == 4 ? a | va << 24 : a;
+        me[(R::kIdx + R::kPat + p) * BLOCK] = W == 4 ? b | vb << 24 : b;
+        if (W == 5) {
+          mb[R::kVal * 4 * BLOCK + p] = (uint8_t)va;
+          mb[(R::kVal + 1) * 4 * BLOCK + p] = (uint8_t)vb;
+        }
+        hr += (int)va;
+        hf += (int)vb;
       }
-      return (int)max(byte_sum(hvr), byte_sum(hvf));
+      return max(hr, hf);
     } else {
-      int s = 0;
+      hr = 0;
+#pragma unroll
       for (int c = 0; c < N; ++c) {
-        int t = tile_at(c);
-        if (!t) continue;
-        int dr = c / W - t / W, dc = c % W - t % W;
-        s += abs(dr) + abs(dc);
+        const int t = mb[4 * BLOCK * (R::kBoard + c / 4) + c % 4];
+        if (t) hr += abs(c / W - t / W) + abs(c % W - t % W);
       }
-      return s;
+      return hr;
     }
   };
   auto set_error = [&](int code, uint32_t info) {
@@ -560,65 +649,71 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
     }
     return false;
   };
-  auto finish_task = [&]() {
-    ++c_done;
-    state = 0;
+  // Add the lane's count to the task's counters.
+  auto flush_count = [&]() {
+    if (!cnt) return;
     if (MULTI) {
-      if (cnt) {
-        // the instance stays in its current iteration while the task is
-        // outstanding; the task's own is that one or, in a pair, the next
-        const uint32_t ci = cur_inst & 0x7FFFFFFFu, tp = cur_inst >> 31;
-        const int cur_iter = ld_volatile(&P.inst_iter[ci]);
-        const int task_iter = cur_iter + (((uint32_t)cur_iter & 1u) != tp ? 1 : 0);
-        atomicAdd(&P.iter_nodes[(size_t)ci * kMaxIters + task_iter], cnt);
-        atomicAdd(&P.sub_loads[(size_t)tp * P.n_subs + sub], cnt);
-      }
+      // the instance stays in its current iteration while the task is
+      // outstanding; the task's own is that one or, in a pair, the next
+      const uint32_t ci = cur_inst & 0x7FFFFFFFu, tp = cur_inst >> 31;
+      const int cur_iter = ld_volatile(&P.inst_iter[ci]);
+      const int task_iter = cur_iter + (((uint32_t)cur_iter & 1u) != tp ? 1 : 0);
+      atomicAdd(&P.iter_nodes[(size_t)ci * kMaxIters + task_iter], (unsigned long long)cnt);
+      atomicAdd(&P.sub_loads[(size_t)tp * P.n_subs + sub], (unsigned long long)cnt);
+    } else {
+      atomicAdd(&P.sub_nodes[sub], (unsigned long long)cnt);
+    }
+    cnt = 0;
+  };
+  auto finish_task = [&]() {
+    atomicAdd(&s_stat[3], 1u);
+    state = 0;
+    flush_count();
+    if (MULTI) {
       __threadfence();
       // the last task of the iteration: the warp advances the instance at the
       // top of its next loop, and only then does this task leave
       // `outstanding`, so that never reads 0 while work is still to come
       if (atomicSub(&P.inst_out[cur_inst & 0x7FFFFFFFu], 1u) == 1u) {
         events |= kAdvance;
-        s_cold[0][tid] = cur_inst & 0x7FFFFFFFu;
+        s_cold0[tid] = cur_inst & 0x7FFFFFFFu;
         return;
       }
-    } else if (cnt) {
-      atomicAdd(&P.sub_nodes[sub], cnt);
     }
     __threadfence();
     atomicSub(&ctl->outstanding, 1u);
   };
   // Copy the claimed record out of its ring slot, then free the slot for the
-  // producer of index slot + cap.
-  auto take_task = [&]() {
+  // producer of index slot + cap.  Returns the task's first-move mask.
+  auto take_task = [&]() -> uint32_t {
     const uint32_t s = slot & (P.cap - 1u);
     const Task *T = &P.tasks[s];
     sub = __ldcg(&T->sub);
     const uint32_t hdr = __ldcg((const uint32_t *)T + 1);
     plen = (int)(hdr & 0xFFFFu);
-    mask0 = (hdr >> 16) & 0xFu;
-    splitk = MULTI ? (int)((hdr >> 24) & 0x3Fu) : (int)(hdr >> 24);
+    splitk = MULTI ? (hdr >> 24) & 0x3Fu : hdr >> 24;
     cur_inst = MULTI ? (hdr << 1) & 0x80000000u : 0u;  // the parity bit until start_task adds the instance
-    for (int wi = 0; wi < kPathWords; ++wi) s_prefix[wi][tid] = __ldcg(&T->path[wi]);
+    for (int wi = 0; 16 * wi < plen; ++wi) prefix[wi] = __ldcg(&T->path[wi]);
     st_release(&P.seq[s], slot + P.cap);  // the copy above completes before the slot is reused
+    return (hdr >> 16) & 0xFu;
   };
-  auto start_task = [&]() -> bool {
-    const SubRoot *R = &P.subs[sub];
-    const uint8_t *rb = R->board;
-    if (W == 4) {
-      uint4 v = *(const uint4 *)rb;
-      const uint8_t *bb = (const uint8_t *)&v;
-      b64 = 0;
-      for (int c = 0; c < 16; ++c) b64 |= (uint64_t)(bb[c] & 15u) << (4 * c);
-    } else {
-      for (int c = 0; c < N; ++c) myboard[c] = rb[c];
+  auto start_task = [&](uint32_t mask0) -> bool {
+    const uint4 *rec = reinterpret_cast<const uint4 *>(&P.subs[sub]);
+    const uint4 b0 = rec[0], b1 = rec[1];
+    me[(R::kBoard + 0) * BLOCK] = b0.x;
+    me[(R::kBoard + 1) * BLOCK] = b0.y;
+    me[(R::kBoard + 2) * BLOCK] = b0.z;
+    me[(R::kBoard + 3) * BLOCK] = b0.w;
+    if (W == 5) {
+      me[(R::kBoard + 4) * BLOCK] = b1.x;
+      me[(R::kBoard + 5) * BLOCK] = b1.y;
+      me[(R::kBoard + 6) * BLOCK] = b1.z;  // cell 24, then the record's blank, g and pre
     }
-    uint4 tailv = *(const uint4 *)(rb + 16);
-    const uint8_t *tb = (const uint8_t *)&tailv;
-    blank = tb[25 - 16];
-    g = tb[26 - 16];
-    pre = tb[27 - 16] == kNoPre ? -1 : (int)tb[27 - 16];
-    uint32_t inst = *(const uint32_t *)(tb + 12);
+    blank = (int)((b1.z >> 8) & 0xFFu);
+    groot = (int)((b1.z >> 16) & 0xFFu);
+    int pre = (b1.z >> 24) == kNoPre ? -1 : (int)(b1.z >> 24);
+    const uint32_t inst = b1.w;
+    int limit;
     if (MULTI) {
       limit = ld_volatile(&P.inst_limit[2 * inst + (cur_inst >> 31)]);
       cur_inst |= inst;
@@ -626,39 +721,43 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
       cur_inst = inst;
       limit = P.inst_limit[inst];
     }
+    boff = board_off(blank);
+    uint32_t word = 0;
     for (int i = 0; i < plen; ++i) {
-      int d = task_dir(i);
-      if (!((legal_moves(W, blank) >> d) & 1u)) {  // corrupt record: never index off the board
+      if ((i & 15) == 0) word = prefix[i >> 4];
+      const uint32_t d = word & 3u;
+      word >>= 2;
+      if (!((step_legal<W>(blank) >> d) & 1u)) {  // corrupt record: never index off the board
         set_error(SP_ERR_ARG, 0x100u + (uint32_t)i);
         return false;
       }
-      int src = blank + move_delta(W, d);
-      slide(tile_at(src), src, blank);
-      blank = src;
-      pre = d;
-      ++g;
+      blank += step_delta<W>(d);
+      const uint32_t foff = board_off(blank);
+      mb[boff] = mb[foff];
+      boff = foff;
+      pre = (int)d;
     }
-    h = full_h();
-    rblank = blank;
-    rpre = pre;
-    groot = g;
-    lo = ((uint32_t)rblank << 8) | ((uint32_t)(rpre + 1) << 16);
+    mb[boff] = 0;
+    groot += plen;
+    const int h = full_h();
+    rem = step_legal<W>(blank) & mask0;
+    if (pre >= 0) rem &= ~(1u << (3 - pre));
+    budget = limit - groot - 1;
+    kstop = splitk ? 0 : min(R::kMaxLev - 1, kMaxPath - plen);
     k = 0;
-    it = 0;
-    top = 0;
-    cut = 0;
+    lo = 0;
     cnt = 0;
-    return g + h <= limit;
+    return groot + h <= limit;
   };
   auto record_goal = [&]() {
     const uint32_t si = P.subs[sub].inst;
     Solution *S = &P.sol[MULTI ? 2 * si + (cur_inst >> 31) : si];
-    atomicMax(&S->best, 0xFFFFFFFFu - (uint32_t)g);  // shortest goal depth over all lanes
+    atomicMax(&S->best, 0xFFFFFFFFu - (uint32_t)(groot + k));  // shortest goal depth over all lanes
     if (atomicCAS(&S->flag, 0u, 1u) == 0u) {
       int len = plen + k;
       S->sub = sub;
       S->len = (uint32_t)len;
-      for (int wi = 0; wi < kPathWords; ++wi) S->path[wi] = path_word(wi, len);
+      write_path(len, [&](int wi, uint32_t w) { S->path[wi] = w; });
       __threadfence();
     }
   };
@@ -668,94 +767,118 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
   // tile into the blank's cell and update the pattern index the same way, so
   // they share one code path (lanes of a warp at different points of their
   // walks stay converged); only the child's table lookups, the f-test and
-  // the stack bookkeeping differ.  Returns true when the task is exhausted.
-  auto step = [&]() -> bool {
-    // minus the reverse of the move into this node: its bit from a nibble
-    // table indexed by pre + 1 (pre = -1 at a task root without one)
-    uint32_t cand = step_legal<W>(blank) & (0xFu << it) & ~((0x12480u >> (4 * (pre + 1))) & 15u);
-    if (k == 0) cand &= mask0;
-    const bool gen = cand != 0;
-    if (!gen && k == 0) return true;
-    int dm;  // the blank's move this step
-    if (gen) {
-      dm = __ffs(cand) - 1;
-    } else {
-      --k;
-      if ((k & 15) == 15) top = s_stack[k >> 4][tid];
-      dm = 3 - (int)((top >> (2 * (k & 15))) & 3u);  // the reverse of the move into level k + 1
-    }
-    const int from = blank + step_delta<W>(dm);
-    const int t = tile_at(from);  // slides from `from` into the blank's cell
-    int nh;
-    uint32_t nhvr = hvr, nhvf = hvf;
-    Idx<W> nir = ir, nif = iff;
-    int pr = 0, pf = 0;
-    if (PDB) {
-      pr = s_pat[t];
-      pf = s_pat[N + t];
-      nir.add(pr, (int32_t)(s_code[t * N + blank] - s_code[t * N + from]));
-      nif.add(pf, (int32_t)(s_code[N * N + t * N + blank] - s_code[N * N + t * N + from]));
-      if (gen || k >= HSAVE) {
-        nhvr = set_byte(hvr, pr, lookup(W == 5 ? (pr != 0) : pr, nir.get(pr)));
-        nhvf = set_byte(hvf, pf, lookup(W == 5 ? (pf != 0) : pf, nif.get(pf)));
+  // the level's word differ.
+  // `mates`: the lanes of the warp that take this step.  The warp syncs keep
+  // them on one path: without them the compiler gives generating and undoing
+  // lanes a copy each of the shared code.
+  // go on; task exhausted; child to hand to the pool; not searching
+  enum { kStepOn, kStepDone, kStepEmit, kStepIdle };
+  auto step = [&](unsigned mates) -> int {
+    const bool gen = rem != 0;
+    // an undo: the level's moves, and the table values it had before the descent
+    uint32_t e = 0, vr = 0, vf = 0;
+    const int lev = gen ? k : k - 1;  // the level whose byte this step writes or reads
+    const uint32_t at = level_off(lev);
+    if (!gen) {
+      if (R::kDeep > 0 && lev >= R::kShared) {
+        const uint32_t w = deep[lev - R::kShared];
+        e = w & 0xFFu;
+        vr = (w >> 8) & 0xFFu;
+        vf = w >> 16;
       } else {
-        const uint32_t sv = s_hsave[k][tid];  // the values this level had before the descent
-        nhvr = set_byte(hvr, pr, sv & 0xFFu);
-        nhvf = set_byte(hvf, pf, sv >> 8);
+        e = mb[at];
+        if (PDB) {
+          vr = mb[at + 4u * BLOCK * R::kPlane];
+          vf = mb[at + 8u * BLOCK * R::kPlane];
+        }
       }
-      nh = (int)max(byte_sum(nhvr), byte_sum(nhvf));
-    } else {
-      nh = h + s_mdd[(dm * N + from) * N + t];
     }
-    if (gen) {
-      ++cnt;
-      if (g + 1 + nh > limit) {  // generated, not entered
-        it = dm + 1;
-        return false;
-      }
-      if (k + 1 >= MAXLEV || plen + k + 1 > kMaxPath) {
-        set_error(SP_ERR_STACK_OVERFLOW, (uint32_t)(plen + k));
-        return true;
-      }
-      if (PDB && k < HSAVE)
-        s_hsave[k][tid] = (uint16_t)(((hvr >> (8 * pr)) & 0xFFu) | (((hvf >> (8 * pf)) & 0xFFu) << 8));
-    }
-    slide(t, from, blank);
-    blank = from;
-    h = nh;
+    __syncwarp(mates);
+    const uint32_t dm = gen ? first_move(rem) : e >> 4;  // the blank's move this step
+    rem &= rem - 1u;
+    cnt += gen;
+    const int from = blank + step_delta<W>(dm);
+    const uint32_t foff = board_off(from);
+    const uint32_t t = mb[foff];  // slides from `from` into the blank's cell
+    uint32_t qr = 0, qf = 0, nr = 0, nf = 0, oldr = 0, oldf = 0, child;
+    int nhr, nhf = 0;
     if (PDB) {
-      ir = nir;
-      iff = nif;
-      hvr = nhvr;
-      hvf = nhvf;
-    }
-    if (gen) {
-      ++g;
-      const int sh = 2 * (k & 15);
-      top = (top & ~(3u << sh)) | ((uint32_t)dm << sh);
-      if ((k & 15) == 15) s_stack[k >> 4][tid] = top;
-      ++k;
-      if (cut && k < 64) cut &= ~(1ull << k);  // cut is almost always 0
-      pre = dm;
-      it = 0;
-      if (nh == 0) record_goal();
-      if (splitk && k == 1) {
-        // split task with `splitk` levels left: this child (already counted
-        // as generated) becomes a task of its own with one level fewer
-        // (published outside the step loop), so a heavy root is split
-        // breadth-first by many lanes; the lane then steps back
-        emit_pending = true;
-        it = 4;
+      if (W == 4) {
+        const uint2 m = s_mv[(t * N + (uint32_t)from) * 4u + dm];
+        qr = m.x & 3u;
+        qf = m.y & 3u;
+        const uint32_t wr = me[(R::kIdx + qr) * BLOCK], wf = me[(R::kIdx + R::kPat + qf) * BLOCK];
+        nr = wr + (uint32_t)((int32_t)m.x >> 8);
+        nf = wf + (uint32_t)((int32_t)m.y >> 8);
+        oldr = wr >> 24;
+        oldf = wf >> 24;
+        child = (m.x >> 4) & 15u;
+      } else {
+        const uint2 ma = s_mv[t * N + (uint32_t)blank], mf = s_mv[t * N + (uint32_t)from];
+        qr = ma.x >> 28;
+        qf = ma.y >> 28;
+        nr = me[(R::kIdx + qr) * BLOCK] + (ma.x - mf.x);
+        nf = me[(R::kIdx + R::kPat + qf) * BLOCK] + (ma.y - mf.y);
+        oldr = mb[R::kVal * 4 * BLOCK + qr];
+        oldf = mb[(R::kVal + 1) * 4 * BLOCK + qf];
+        child = s_rem[(uint32_t)from * 4u + dm];
       }
+      if (gen) {
+        vr = lookup(W == 4 ? nr & 0x3FFFFFu : nr);
+        vf = lookup(W == 4 ? nf & 0x3FFFFFu : nf);
+      }
+      __syncwarp(mates);
+      nhr = hr + (int)(vr - oldr);
+      nhf = hf + (int)(vf - oldf);
     } else {
-      --g;
-      it = (3 - dm) + 1;  // the next sibling of the undone move
-      if (cut && k < 64 && ((cut >> k) & 1ull)) it = 4;
-      if (k == 0) pre = rpre;
-      else if (k & 15) pre = (int)((top >> (2 * ((k - 1) & 15))) & 3u);
-      else pre = (int)((s_stack[(k - 1) >> 4][tid] >> 30) & 3u);
+      const uint32_t m = s_md[(t * N + (uint32_t)from) * 4u + dm];
+      child = m & 15u;
+      nhr = hr + (int)((m >> 3) & 2u) - 1;
     }
-    return false;
+    const int nh = PDB ? max(nhr, nhf) : nhr;
+    int ev = kStepOn;
+    if (!gen || nh <= budget - k) {  // else: generated, not entered
+      if (PDB) {
+        me[(R::kIdx + qr) * BLOCK] = W == 4 ? nr + ((vr - oldr) << 24) : nr;
+        me[(R::kIdx + R::kPat + qf) * BLOCK] = W == 4 ? nf + ((vf - oldf) << 24) : nf;
+        if (W == 5) {
+          mb[R::kVal * 4 * BLOCK + qr] = (uint8_t)vr;
+          mb[(R::kVal + 1) * 4 * BLOCK + qf] = (uint8_t)vf;
+        }
+        hf = nhf;
+      }
+      hr = nhr;
+      mb[boff] = (uint8_t)t;
+      boff = foff;
+      blank = from;
+      if (gen) {
+        const uint32_t up = rem | (3u - dm) << 4;
+        if (R::kDeep > 0 && lev >= R::kShared) {
+          deep[lev - R::kShared] = up | oldr << 8 | oldf << 16;
+        } else {
+          mb[at] = (uint8_t)up;
+          if (PDB) {
+            mb[at + 4u * BLOCK * R::kPlane] = (uint8_t)oldr;
+            mb[at + 8u * BLOCK * R::kPlane] = (uint8_t)oldf;
+          }
+        }
+        ++k;
+        rem = child;
+        if (nh == 0) record_goal();
+        if (lev == kstop) {
+          // split task with `splitk` levels left: this child (already counted
+          // as generated) becomes a task of its own with one level fewer
+          // (published outside the step loop), so a heavy root is split
+          // breadth-first by many lanes; the lane then steps back
+          ev = splitk ? kStepEmit : kStepDone;
+          if (!splitk) set_error(SP_ERR_STACK_OVERFLOW, (uint32_t)(plen + lev));
+        }
+      } else {
+        --k;
+        rem = e & 15u;
+      }
+    }
+    return ev;
   };
 
   // Give the untried moves of the shallowest open level (slack >= min_slack)
@@ -763,39 +886,20 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
   auto find_donation = [&](uint32_t &mask_out) -> int {
     // resume at the first level not yet seen exhausted (`lo`): a level only
     // loses untried moves during a task, so the walk never needs to look
-    // below it again; above the current depth the cache restarts at k
-    int j = (int)(lo & 0xFFu), bl = (int)((lo >> 8) & 0xFFu), pr = (int)((lo >> 16) & 7u) - 1;
-    if (k < j) {
-      j = k;
-      bl = blank;
-      pr = pre;
-    }
-    const int lim = min(k, 63);
-    int found = -1;
-    for (; j <= lim; ++j) {
-      if (limit - (groot + j) < P.min_slack) break;
-      const int dj = j == k ? 0 : stack_dir(j);
-      uint32_t un = legal_moves(W, bl) & (j == k ? (0xFu << it) : ((0xFu << (dj + 1)) & 0xFu));
-      if (pr >= 0) un &= ~(1u << (3 - pr));
-      if (j == 0) un &= mask0;
-      if (!((cut >> j) & 1ull) && un) {
+    // below it again; above the current depth it restarts at k
+    int j = min(lo, k), found = -1;
+    const int last = min(k, budget + 1 - P.min_slack);
+    for (; j <= last; ++j) {
+      const uint32_t un = j == k ? rem : level_get(j) & 15u;
+      if (un) {
         mask_out = un;
         found = j;
         break;
       }
-      if (j == k) break;
-      bl += move_delta(W, dj);
-      pr = dj;
     }
-    lo = (uint32_t)min(j, 255) | ((uint32_t)bl << 8) | ((uint32_t)(pr + 1) << 16);
+    lo = min(j, k);
     return found;
   };
-
-  unsigned long long last_change = 0;
-  uint32_t last_out = 0xFFFFFFFFu, last_tail = 0xFFFFFFFFu, last_hb = 0xFFFFFFFFu, beat = 0;
-  unsigned backoff = 256;  // idle-warp sleep, ns, doubled up to SP_MAX_BACKOFF_NS
-  unsigned long long c_steps = 0, c_slots = 0, c_idle = 0;
-  const long long t_begin = clock64();
 
   for (;;) {
     const long long t_iter = clock64();
@@ -805,7 +909,7 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
       while (pend) {
         const int src = __ffs(pend) - 1;
         pend &= pend - 1u;
-        warp_advance(P, s_cold[0][(tid & ~31) + src], s_hist[tid >> 5]);
+        warp_advance(P, s_cold0[(tid & ~31) + src], s_hist[tid >> 5]);
         if (lane == src) {
           events &= ~kAdvance;
           __threadfence();
@@ -813,10 +917,10 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
         }
       }
     }
-    if ((events & kDebt) && ld_acquire(&P.seq[s_cold[1][tid] & (P.cap - 1u)]) == s_cold[1][tid]) {
-      const uint32_t debt = s_cold[1][tid];
+    if ((events & kDebt) && ld_acquire(&P.seq[s_cold1[tid] & (P.cap - 1u)]) == s_cold1[tid]) {
+      const uint32_t debt = s_cold1[tid];
       Task *D = &P.tasks[debt & (P.cap - 1u)];
-      D->sub = s_cold[2][tid];
+      D->sub = s_cold2[tid];
       D->plen = 0;
       D->mask = 0;  // no first move: the claimant finishes it at once
       D->flags = 0;
@@ -865,8 +969,8 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
     // 2. a claimed index becomes a task once its producer published it; only
     //    indices already reserved (below the cached tail) are polled
     if (state == 1 && slot < tl && ld_acquire(&P.seq[slot & (P.cap - 1u)]) == slot + 1u) {
-      take_task();
-      if (start_task()) state = 2;
+      const uint32_t mask0 = take_task();
+      if (start_task(mask0)) state = 2;
       else finish_task();
     }
     // 3. nobody in the warp is searching: finished, failed or waiting
@@ -875,37 +979,53 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
       if (out == 0) break;
       if (lane == 0) {
         const unsigned long long now = globaltimer();
-        if (out != last_out || tl != last_tail || hb != last_hb || last_change == 0) {
-          last_out = out;
-          last_tail = tl;
-          last_hb = hb;
-          last_change = now;
-        } else if (now - last_change > P.timeout_ns) {
+        if (out != ws.last_out || tl != ws.last_tail || hb != ws.last_hb || ws.last_change == 0) {
+          ws.last_out = out;
+          ws.last_tail = tl;
+          ws.last_hb = hb;
+          ws.last_change = now;
+        } else if (now - ws.last_change > P.timeout_ns) {
           set_error(SP_ERR_TIMEOUT, out);
         }
       }
+      const unsigned backoff = ws.backoff;  // doubled up to SP_MAX_BACKOFF_NS
       __nanosleep(backoff);
-      backoff = min(backoff * 2u, (unsigned)SP_MAX_BACKOFF_NS);
-      c_idle += (unsigned long long)(clock64() - t_iter);
+      __syncwarp();
+      if (lane == 0) {
+        ws.backoff = min(backoff * 2u, (unsigned)SP_MAX_BACKOFF_NS);
+        ws.idle += (unsigned long long)(clock64() - t_iter);
+      }
+      __syncwarp();
       continue;
     }
-    backoff = 256;
-    last_change = 0;  // a new idle spell starts its own no-progress clock
-    if (lane == 0 && ((++beat & 127u) == 0u)) atomicAdd(&ctl->heartbeat, 1u);
+    if (lane == 0) {
+      ws.backoff = 256;
+      ws.last_change = 0;  // a new idle spell starts its own no-progress clock
+      if ((++ws.beat & 127u) == 0u) atomicAdd(&ctl->heartbeat, 1u);
+    }
     // 4. search
-    c_slots += 32ull * (unsigned long long)P.steps;
-    if (state == 2) {
-      bool fin = false;
-      for (int s = 0; s < P.steps; ++s) {
-        ++c_steps;
-        if (step()) {
-          fin = true;
-          break;
-        }
-        if (emit_pending) break;
+    // the warp steps together: every lane stays in the loop until none
+    // searches, and the vote brings them back together
+    int ev = state == 2 ? kStepOn : kStepIdle;
+    uint32_t taken = 0;
+    for (int s = 0; s < P.steps; ++s) {
+      const bool go = ev == kStepOn && (rem | (uint32_t)k) != 0u;  // else: nothing left of the task
+      const unsigned mates = __ballot_sync(FULL, go);
+      if (!mates) break;
+      if (go) {
+        ++taken;
+        ev = step(mates);
       }
-      if (emit_pending) {
-        emit_pending = false;
+    }
+    if (ev == kStepOn && (rem | (uint32_t)k) == 0u) ev = kStepDone;
+    taken = __reduce_add_sync(FULL, taken);
+    if (lane == 0) {
+      ws.slots += 32ull * (unsigned long long)P.steps;
+      ws.steps += taken;
+    }
+    if (state == 2) {
+      if (cnt >= (1u << 30)) flush_count();  // long before the 32-bit count wraps
+      if (ev == kStepEmit) {
         // the split is advisory: with a debt outstanding or the ring half
         // full, the lane searches the subtree itself
         bool emitted = false;
@@ -920,19 +1040,19 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
             D->plen = (uint16_t)len;
             D->mask = 0xF;
             D->flags = (uint8_t)((splitk - 1) | (MULTI ? (cur_inst >> 31) << 6 : 0u));
-            for (int wi = 0; wi < kPathWords; ++wi) D->path[wi] = path_word(wi, len);
+            write_path(len, [&](int wi, uint32_t w) { D->path[wi] = w; });
             st_release(&P.seq[t & (P.cap - 1u)], t + 1u);
             emitted = true;
           } else {
-            ++c_notfree;
+            atomicAdd(&s_stat[1], 1u);
             events |= kDebt;
-            s_cold[1][tid] = t;
-            s_cold[2][tid] = sub;
+            s_cold1[tid] = t;
+            s_cold2[tid] = sub;
           }
         }
-        if (!emitted) it = 0;
+        if (emitted) rem = 0;
       }
-      if (fin) finish_task();
+      if (ev == kStepDone) finish_task();
     }
     // 5. donate while fewer than `reserve` tasks are queued (tail - head)
     if (P.donate && hd + P.reserve > tl) {
@@ -950,8 +1070,8 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
       const bool donor = ((cand >> lane) & 1u) && rank < allowed && !(events & kDebt);
       const unsigned donors = __ballot_sync(FULL, donor);
       if (lane == 0) {
-        ++c_nowait;  // hungry polls
-        if (donors) ++c_found;
+        atomicAdd(&s_stat[2], 1u);  // hungry polls
+        if (donors) atomicAdd(&s_stat[4], 1u);
       }
       uint32_t tbase = 0;
       const int lead = donors ? __ffs(donors) - 1 : 0;
@@ -966,15 +1086,15 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
         // in practice it already is -- wait a bounded time, else keep the
         // branch and owe the index a null task
         const uint32_t mask = P.cap - 1u;
-        ++c_tries;
+        atomicAdd(&s_stat[0], 1u);
         if (MULTI) atomicAdd(&P.inst_out[cur_inst & 0x7FFFFFFFu], 1u);  // the donor's own task keeps it >= 1
         const uint32_t t = tbase + (uint32_t)__popc(donors & ((1u << lane) - 1u));
         const bool ok = slot_free(t, 4096);
         if (!ok) {
-          ++c_notfree;
+          atomicAdd(&s_stat[1], 1u);
           events |= kDebt;
-          s_cold[1][tid] = t;
-          s_cold[2][tid] = sub;
+          s_cold1[tid] = t;
+          s_cold2[tid] = sub;
         }
         if (ok) {
           Task *D = &P.tasks[t & mask];
@@ -983,36 +1103,24 @@ __global__ void __launch_bounds__(BLOCK, SP_SEARCH_THREADS_PER_SM / BLOCK) searc
           D->plen = (uint16_t)nlen;
           D->mask = (uint8_t)dmask;
           D->flags = (uint8_t)(MULTI ? (cur_inst >> 31) << 6 : 0u);
-          for (int wi = 0; wi < kPathWords; ++wi) D->path[wi] = path_word(wi, nlen);
+          write_path(nlen, [&](int wi, uint32_t w) { D->path[wi] = w; });
           st_release(&P.seq[t & mask], t + 1u);
           atomicAdd(&ctl->donated, 1ull);
-          if (lev == k) it = 4;
-          else cut |= 1ull << lev;
+          if (lev == k) rem = 0;
+          else level_cut(lev);
         }
       }
     }
   }
-  // efficiency counters (warp-aggregated)
-  unsigned long long steps_w = c_steps, tries_w = c_tries, notfree_w = c_notfree, nowait_w = c_nowait,
-                     done_w = c_done;
-  for (int o = 16; o; o >>= 1) {
-    steps_w += __shfl_xor_sync(FULL, steps_w, o);
-    tries_w += __shfl_xor_sync(FULL, tries_w, o);
-    notfree_w += __shfl_xor_sync(FULL, notfree_w, o);
-    nowait_w += __shfl_xor_sync(FULL, nowait_w, o);
-    done_w += __shfl_xor_sync(FULL, done_w, o);
-  }
+  // efficiency counters
   if (lane == 0) {
-    atomicAdd(&ctl->counters[0], steps_w);
-    atomicAdd(&ctl->counters[1], c_slots);
-    atomicAdd(&ctl->counters[2], c_idle);
-    atomicAdd(&ctl->counters[3], (unsigned long long)(clock64() - t_begin));
-    atomicAdd(&ctl->counters[4], tries_w);
-    atomicAdd(&ctl->counters[5], notfree_w);
-    atomicAdd(&ctl->counters[6], nowait_w);
-    atomicAdd(&ctl->counters[7], done_w);
-    atomicAdd(&ctl->counters[8], c_found);
+    atomicAdd(&ctl->counters[0], ws.steps);
+    atomicAdd(&ctl->counters[1], ws.slots);
+    atomicAdd(&ctl->counters[2], ws.idle);
+    atomicAdd(&ctl->counters[3], (unsigned long long)clock64() - ws.begin);
   }
+  __syncthreads();
+  if (tid < 5) atomicAdd(&ctl->counters[4 + tid], (unsigned long long)s_stat[tid]);
 }
 
 // Reset the ring (seq[s] = s: slot s free for index s), fill indices [0, n)

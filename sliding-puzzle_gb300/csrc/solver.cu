@@ -329,7 +329,13 @@ void build_heur_tables(int w, HeurTables *ht) {
         uint32_t mul = 1;
         for (int q = j + 1; q < ps.k; ++q) mul *= (uint32_t)ps.radix;
         ht->pat[part][tile] = (uint8_t)p;
-        for (int c = 0; c < n; ++c) ht->code[part][tile * n + c] = (uint32_t)sym_cell(w, sym, c) * mul;
+        for (int c = 0; c < n; ++c) {
+          const uint32_t code = (uint32_t)sym_cell(w, sym, c) * mul;
+          const int i = tile * n + c;
+          ht->code[part][i] = code;
+          if (w == 4) ht->sum[2 * i + part] = (uint64_t)code << (20 * p);
+          else ht->sum[4 * i + 2 * part + (p >> 1)] = (uint64_t)code << (28 * (p & 1));
+        }
       }
     }
   }

@@ -150,6 +150,11 @@ struct HeurTables {
   uint8_t pat[2][kMaxN];            // [part][tile] -> pattern (0xFF for the blank)
   int8_t mdd[4 * kMaxN * kMaxN];    // [(d*N + cell)*N + tile]: MD change when the tile at
                                     // `cell` slides into the blank after the blank's move d
+  // Pattern indices of a board as plain sums: per (tile, cell) its digit
+  // contributions shifted to the fields of packed index words, 0 for the
+  // blank.  Width 4: {regular, reflected}, three 20-bit fields each; width 5:
+  // {regular 0-1, regular 2-3, reflected 0-1, reflected 2-3}, 28-bit fields.
+  alignas(16) uint64_t sum[kMaxN * kMaxN * 4];
 };
 
 }  // namespace sp
