@@ -14,15 +14,15 @@
 //     region of its home cell 0;
 //   * a table entry is the distance to the goal, minimised over the blank's
 //     regions (the reference's index holds no blank position).
-// The search runs level-synchronously over a [placement rank][region]
-// byte array (placement rank = lexicographic rank of the k-permutation of
-// cells, the byte order of the reference's table files), one thread per
-// placement row per level.  Rows are 16 or 32 bytes (one byte per possible
-// lowest cell of a region) so a row is read with one or two 16-byte loads.
+// The search runs level by level over the abstract states themselves: a queue
+// of (placement, region) entries, each appended once, whose slice [bounds[d],
+// bounds[d + 1]) is level d.  The regions of a placement depend only on which
+// cells are occupied, so a table over the C(n, k) subsets gives every cell's
+// region number (at most 5), and one visited bit per region makes 64 MB of a
+// 6-tile table's 181 M states: it stays in L2.  A placement's first visit
+// writes its entry straight into the lookup layout.
 #include <cuda_runtime.h>
 #include <stdint.h>
-
-#include <chrono>
 
 #include "sp_defs.h"
 #include "sp_device.cuh"
@@ -32,157 +32,323 @@ namespace sp {
 
 namespace {
 
-struct Geo {
-  int w, n, k;
-  uint32_t full, not_col0, not_collast;
-  int base[6];
-};
-
-Geo make_geo(int w, int table_id) {
-  Geo g{};
-  g.w = w;
-  g.n = w * w;
-  PatternSet ps = pattern_set(w);
-  g.k = ps.k;
-  g.full = (1u << g.n) - 1u;
-  uint32_t c0 = 0, cl = 0;
-  for (int r = 0; r < w; ++r) {
-    c0 |= 1u << (r * w);
-    cl |= 1u << (r * w + w - 1);
-  }
-  g.not_col0 = g.full & ~c0;
-  g.not_collast = g.full & ~cl;
-  for (int j = 0; j < g.k; ++j) g.base[j] = ps.table_tiles[table_id][j];
-  return g;
+// n choose k for the subset numbers.
+constexpr uint32_t choose(int n, int k) {
+  uint64_t r = 1;
+  for (int i = 0; i < k; ++i) r = r * (uint64_t)(n - i) / (uint64_t)(i + 1);
+  return n < k ? 0u : (uint32_t)r;
 }
 
-__host__ __device__ __forceinline__ uint32_t flood(const Geo &g, uint32_t free_cells, int c) {
-  uint32_t r = 1u << c, prev;
+template <int W>
+struct Geo {
+  static constexpr int N = W * W, K = W == 5 ? 6 : 5;
+  static constexpr uint32_t kFull = (1u << N) - 1u;
+  static constexpr int kLoBits = (N + 1) / 2;  // a cell mask in two halves, for its subset number
+  static constexpr uint32_t kSubsets = choose(N, K);
+  static constexpr uint32_t kSubsetWords = (kSubsets + 31) / 32;
+  // cells of one column
+  static constexpr uint32_t column(int c) {
+    uint32_t m = 0;
+    for (int r = 0; r < W; ++r) m |= 1u << (r * W + c);
+    return m;
+  }
+  // weight of digit i of a placement's rank / of its lookup index
+  static constexpr uint32_t rank_weight(int i) {
+    uint32_t w = 1;
+    for (int m = i + 1; m < K; ++m) w *= (uint32_t)(N - m);
+    return w;
+  }
+  static constexpr uint32_t index_weight(int i) {
+    uint32_t w = 1;
+    for (int m = i + 1; m < K; ++m) w *= (uint32_t)N;
+    return w;
+  }
+};
+
+template <int W>
+__host__ __device__ __forceinline__ uint32_t flood(uint32_t free_cells, uint32_t from) {
+  using G = Geo<W>;
+  uint32_t r = from, prev;
   do {
     prev = r;
-    r = (r | ((r << 1) & g.not_col0) | ((r >> 1) & g.not_collast) | (r << g.w) | (r >> g.w)) &
-        free_cells;
+    r = (r | ((r << 1) & ~G::column(0)) | ((r >> 1) & ~G::column(W - 1)) | (r << W) | (r >> W)) & free_cells;
   } while (r != prev);
   return r;
 }
 
-__host__ __device__ __forceinline__ int neighbour(const Geo &g, int cell, int d) {
-  int r = cell / g.w, c = cell - r * g.w;
-  switch (d) {
-    case 0: return r == 0 ? -1 : cell - g.w;
-    case 1: return c == g.w - 1 ? -1 : cell + 1;
-    case 2: return c == 0 ? -1 : cell - 1;
-    default: return r == g.w - 1 ? -1 : cell + g.w;
+// Cells of placement `rank` (lexicographic rank of the k-permutation of
+// cells, the byte order of the reference's table files): the digits by
+// constant divisions, each then moved past the cells used before it, which
+// are kept sorted.
+template <int W>
+__device__ __forceinline__ void unrank(uint32_t rank, int (&pos)[Geo<W>::K]) {
+  using G = Geo<W>;
+  int sorted[G::K];
+#pragma unroll
+  for (int i = G::K - 1; i >= 0; --i) {
+    const uint32_t q = rank / (uint32_t)(G::N - i);
+    pos[i] = (int)(rank - q * (uint32_t)(G::N - i));
+    rank = q;
+  }
+#pragma unroll
+  for (int i = 0; i < G::K; ++i) {
+    int p = pos[i];
+#pragma unroll
+    for (int m = 0; m < i; ++m) p += p >= sorted[m];
+    pos[i] = p;
+    sorted[i] = p;
+#pragma unroll
+    for (int m = i; m > 0; --m) {
+      const int lo = min(sorted[m - 1], sorted[m]), hi = max(sorted[m - 1], sorted[m]);
+      sorted[m - 1] = lo;
+      sorted[m] = hi;
+    }
   }
 }
 
-__host__ __device__ __forceinline__ uint64_t rank_k(int n, int k, const int *pos) {
-  uint64_t r = 0;
-  uint32_t used = 0;
-  for (int i = 0; i < k; ++i) {
-#ifdef __CUDA_ARCH__
-    int less = __popc(used & ((1u << pos[i]) - 1u));
-#else
-    int less = __builtin_popcount(used & ((1u << pos[i]) - 1u));
-#endif
-    r = r * (uint64_t)(n - i) + (uint64_t)(pos[i] - less);
-    used |= 1u << pos[i];
-  }
-  return r;
-}
-
-__device__ __forceinline__ void unrank_k(int n, int k, uint64_t r, int *pos) {
-  int digit[6];
-  for (int i = k - 1; i >= 0; --i) {
-    uint64_t q = r / (uint64_t)(n - i);
-    digit[i] = (int)(r - q * (uint64_t)(n - i));
-    r = q;
-  }
-  uint32_t unused = (1u << n) - 1u;
-  for (int i = 0; i < k; ++i) {
-    // position of the (digit+1)-th set bit of `unused`
-    uint32_t m = unused;
-    for (int s = 0; s < digit[i]; ++s) m &= m - 1u;
-    int c = __ffs(m) - 1;
-    pos[i] = c;
-    unused &= ~(1u << c);
-  }
-}
-
-__device__ __forceinline__ uint32_t lookup_index(int n, int k, const int *pos) {
+template <int W>
+__device__ __forceinline__ uint32_t lookup_index(const int (&pos)[Geo<W>::K]) {
   uint32_t x = 0;
-  for (int j = 0; j < k; ++j) x = x * (uint32_t)n + (uint32_t)pos[j];
+#pragma unroll
+  for (int j = 0; j < Geo<W>::K; ++j) x = x * (uint32_t)Geo<W>::N + (uint32_t)pos[j];
   return x;
 }
 
-constexpr uint8_t kUnseen = 0xFF;
+// Per-build tables: the subset number of a k-cell mask is the sum of its low
+// half's entry and its high half's (their colexicographic numbers; the high
+// half's cells come after the k - popc(high) low ones), and per subset the
+// region number of every free cell as three bit planes (regions in the order
+// of their lowest cells), the number of regions in w.  `split`: a bit per
+// subset with more than one region.
+struct SubsetTables {
+  uint16_t *lo;
+  uint32_t *hi, *split;
+  uint4 *regions;
+};
 
-template <int STRIDE>
-__global__ void bfs_level_kernel(uint8_t *dist, uint64_t T, Geo g, int d,
-                                 unsigned long long *produced) {
-  unsigned long long local = 0;
-  const uint32_t dd = 0x01010101u * (uint32_t)d;
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < T;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    uint8_t *row = dist + r * STRIDE;
-    uint4 v[STRIDE / 16];
+template <int W>
+__global__ void subset_kernel(SubsetTables S, unsigned long long *n_regions) {
+  using G = Geo<W>;
+  auto colex = [](uint32_t mask, int base, int first) -> uint32_t {  // i-th set bit p -> C(base + p, first + i)
+    uint32_t r = 0;
+    for (int i = first; mask; mask &= mask - 1u) {
+      ++i;
+      const int n = base + __ffs(mask) - 1;
+      uint64_t c = 1;
+      for (int q = 0; q < i; ++q) c = c * (uint64_t)(n - q) / (uint64_t)(q + 1);
+      r += n < i ? 0u : (uint32_t)c;
+    }
+    return r;
+  };
+  const uint32_t mask = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t hi = mask >> G::kLoBits, lo = mask & ((1u << G::kLoBits) - 1u);
+  if (hi == 0 && __popc(lo) <= G::K) S.lo[lo] = (uint16_t)colex(lo, 0, 0);
+  if (lo == 0 && __popc(hi) <= G::K) S.hi[hi] = colex(hi, G::kLoBits, G::K - __popc(hi));
+  if (mask > G::kFull || __popc(mask) != G::K) return;
+  const uint32_t sub = colex(mask, 0, 0);
+  uint32_t free_cells = G::kFull & ~mask, n = 0;
+  uint4 v = make_uint4(0, 0, 0, 0);
+  while (free_cells) {
+    const uint32_t r = flood<W>(G::kFull & ~mask, free_cells & (0u - free_cells));
+    free_cells &= ~r;
+    if (n & 1u) v.x |= r;
+    if (n & 2u) v.y |= r;
+    if (n & 4u) v.z |= r;
+    ++n;
+  }
+  v.w = n;
+  S.regions[sub] = v;
+  if (n > 1) atomicOr(S.split + sub / 32, 1u << (sub % 32));
+  atomicAdd(n_regions, (unsigned long long)n);
+}
+
+// One table's search.
+struct BfsArgs {
+  SubsetTables subsets;
+  uint32_t *queue;    // rank << 3 | region of every state, in the order found
+  uint32_t cap;       // its entries: the number of states
+  uint32_t *visited;  // regions 0-3 of a placement: a nibble
+  uint32_t *extra;    // region 4: a bit
+  uint8_t *lookup;
+  uint32_t *bounds;   // level d: queue[bounds[d] .. bounds[d + 1])
+  uint32_t *tail;     // entries in the queue
+  uint32_t *done;     // blocks of this level that have finished
+  uint32_t goal;      // lookup index of the goal
+};
+
+struct Goal {
+  uint32_t rank, region, index;
+};
+
+__global__ void bfs_start_kernel(BfsArgs A, Goal g) {
+  A.queue[0] = g.rank << 3 | g.region;
+  A.visited[g.rank >> 3] = 1u << (4 * (g.rank & 7u) + g.region);  // the blank's home region is number 0..3
+  A.lookup[g.index] = 0;
+  A.bounds[0] = 0;
+  A.bounds[1] = 1;
+  *A.tail = 1;
+  *A.done = 0;
+}
+
+// Expand level d: a lane takes a state, its warp tries the K * 4 moves in
+// turn, four at a time with their reads and then their atomics in flight
+// together (2.9 ms; one at a time 3.1), tests a child's visited bit by a
+// plain read first -- 9 in 10 were seen before -- and appends what is new to
+// the queue through a buffer of the warp, one reservation per 128-256
+// entries.  A child's rank and lookup index
+// differ from its parent's by constants, except that a vertical move also
+// passes up to W - 1 occupied cells.
+// Bound by its reads of the visited bits (64 MB) and, where the occupied
+// cells divide the board (37 % of the subsets), of the region table (2.8 MB),
+// all in L2, at half of the issue slots: the largest level of a 6-tile table
+// (21 M states, 225 M children) takes 2.9 ms, 181 G L2 sectors/s.  Both
+// 24-puzzle tables 546 -> 52 ms, the three 15-puzzle ones 6.1 -> 1.7 ms.
+// The version before it scanned a [placement][region]
+// byte array of 4.1 GB per level, expanded the 1-3 hits of a warp in turn and
+// waited for the host after each level.
+constexpr int kBfsBlock = 512;
+constexpr uint32_t kBfsBuf = 256;
+template <int W>
+__global__ void __launch_bounds__(kBfsBlock) bfs_level_kernel(BfsArgs A, int d) {
+  using G = Geo<W>;
+  constexpr int N = G::N, K = G::K;
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ uint32_t s_hi[1u << (N - G::kLoBits)], s_split[G::kSubsetWords];
+  __shared__ uint16_t s_lo[1u << G::kLoBits];
+  __shared__ uint32_t s_buf[kBfsBlock / 32][kBfsBuf];
+  const uint32_t s0 = A.bounds[d], s1 = A.bounds[d + 1];
+  if (s0 == s1) {  // an empty level: the search is over
+    if (blockIdx.x == 0 && threadIdx.x == 0) A.bounds[d + 2] = s1;
+    return;
+  }
+  for (uint32_t i = threadIdx.x; i < (1u << G::kLoBits); i += kBfsBlock) s_lo[i] = __ldg(A.subsets.lo + i);
+  for (uint32_t i = threadIdx.x; i < (1u << (N - G::kLoBits)); i += kBfsBlock) s_hi[i] = __ldg(A.subsets.hi + i);
+  for (uint32_t i = threadIdx.x; i < G::kSubsetWords; i += kBfsBlock) s_split[i] = __ldg(A.subsets.split + i);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  uint32_t *buf = s_buf[threadIdx.x >> 5];
+  uint32_t n_buf = 0;  // the same in all lanes
+  auto flush = [&]() {
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(A.tail, n_buf);
+    at = __shfl_sync(FULL, at, 0);
+    for (uint32_t i = lane; i < n_buf; i += 32)
+      if (at + i < A.cap) A.queue[at + i] = buf[i];
+    __syncwarp();
+    n_buf = 0;
+  };
+  auto subset = [&](uint32_t mask) -> uint32_t {
+    return s_lo[mask & ((1u << G::kLoBits) - 1u)] + s_hi[mask >> G::kLoBits];
+  };
+  const uint32_t warps = gridDim.x * (kBfsBlock / 32), warp = (blockIdx.x * kBfsBlock + threadIdx.x) >> 5;
+  // a small level is spread over K times as many warps, a tile each
+  const uint32_t packs = (s1 - s0 + 31) / 32;
+  const bool spread = packs * K <= warps;
+  const int only = spread ? (int)(warp % K) : -1;
+  for (uint32_t pack = spread ? warp / K : warp; pack < packs; pack += warps) {
+    const uint32_t base = s0 + 32 * pack;
+    const bool valid = base + lane < s1;
+    const uint32_t ent = valid ? A.queue[base + lane] : 0u;
+    const uint32_t rank = ent >> 3;
+    int pos[K];
+    unrank<W>(rank, pos);
+    const uint32_t index = lookup_index<W>(pos);
+    uint32_t mask = 0;
 #pragma unroll
-    for (int q = 0; q < STRIDE / 16; ++q) v[q] = *(const uint4 *)(row + 16 * q);
-    uint32_t hit = 0;
+    for (int j = 0; j < K; ++j) mask |= 1u << pos[j];
+    const uint4 e = __ldg(A.subsets.regions + subset(mask));
+    uint32_t reg = valid ? G::kFull & ~mask : 0u;  // cells of the blank's region
+    reg &= ent & 1u ? e.x : ~e.x;
+    reg &= ent & 2u ? e.y : ~e.y;
+    reg &= ent & 4u ? e.z : ~e.z;
+    // bit p set: the tile on cell p can move that way into the region
+    const uint32_t can[4] = {reg << W, (reg & ~G::column(0)) >> 1, (reg & ~G::column(W - 1)) << 1, reg >> W};
+    uint32_t earlier = 0;  // cells of the tiles before j
 #pragma unroll
-    for (int q = 0; q < STRIDE / 16; ++q)
-      hit |= __vcmpeq4(v[q].x, dd) | __vcmpeq4(v[q].y, dd) | __vcmpeq4(v[q].z, dd) |
-             __vcmpeq4(v[q].w, dd);
-    if (!hit) continue;
-    const uint8_t *rb = (const uint8_t *)v;
-    int pos[6] = {0, 0, 0, 0, 0, 0};
-    unrank_k(g.n, g.k, r, pos);
-    uint32_t occ = 0;
-    for (int j = 0; j < g.k; ++j) occ |= 1u << pos[j];
-    const uint32_t free_cells = g.full & ~occ;
-    for (int m = 0; m < g.n; ++m) {
-      if (rb[m] != d) continue;
-      const uint32_t reg = flood(g, free_cells, m);
-      for (int j = 0; j < g.k; ++j) {
-        for (int dir = 0; dir < 4; ++dir) {
-          const int c = neighbour(g, pos[j], dir);
-          if (c < 0 || !((reg >> c) & 1u)) continue;
-          int q[6];
-          for (int a = 0; a < 6; ++a) q[a] = pos[a];
-          q[j] = c;
-          const uint32_t free2 = (free_cells & ~(1u << c)) | (1u << pos[j]);
-          const uint32_t reg2 = flood(g, free2, pos[j]);
-          const uint64_t r2 = rank_k(g.n, g.k, q);
-          uint8_t *e = dist + r2 * STRIDE + (__ffs(reg2) - 1);
-          if (*e == kUnseen) {
-            *e = (uint8_t)(d + 1);
-            ++local;
+    for (int j = 0; j < K; ++j) {
+      const int p = pos[j];
+      if (only >= 0 && only != j) {
+        earlier |= 1u << p;
+        continue;
+      }
+      constexpr int step[4] = {-W, 1, -1, W};
+      // the tile's four moves: their reads first, all in flight together
+      uint4 ce[4];
+      uint32_t r2[4], word[4];
+#pragma unroll
+      for (int dir = 0; dir < 4; ++dir) {
+        ce[dir] = make_uint4(0, 0, 0, 0);
+        r2[dir] = word[dir] = 0;
+        if ((can[dir] >> p) & 1u) {
+          const int c = p + step[dir];
+          const uint32_t sub = subset(mask ^ (1u << p) ^ (1u << c));
+          if ((s_split[sub / 32] >> (sub % 32)) & 1u) ce[dir] = __ldg(A.subsets.regions + sub);  // else region 0
+          int change = step[dir];  // of digit j: the cells passed, less those of earlier tiles
+          int32_t later = 0;       // of the later digits: one more tile before them, or one less
+          if (dir == 0 || dir == 3) {
+            const uint32_t passed = mask & (((1u << (W - 1)) - 1u) << (min(p, c) + 1));
+            const int nb = __popc(passed & earlier);
+            change += dir == 3 ? -nb : nb;
+#pragma unroll
+            for (int i = j + 1; i < K; ++i)
+              if ((passed >> pos[i]) & 1u) later += (int32_t)G::rank_weight(i);
+            if (dir == 0) later = -later;
           }
+          r2[dir] = rank + (uint32_t)(change * (int32_t)G::rank_weight(j) + later);
+          word[dir] = __ldcg(A.visited + (r2[dir] >> 3));
         }
       }
+      // then the bits of the unseen children, again in flight together
+      uint32_t region[4], old[4];
+#pragma unroll
+      for (int dir = 0; dir < 4; ++dir) {
+        region[dir] = ((ce[dir].x >> p) & 1u) | ((ce[dir].y >> p) & 1u) << 1 | ((ce[dir].z >> p) & 1u) << 2;
+        const uint32_t bit = 4 * (r2[dir] & 7u) + region[dir];
+        old[dir] = 0xFFFFFFFFu;
+        if ((can[dir] >> p) & 1u) {
+          if (region[dir] > 3) old[dir] = atomicOr(A.extra + (r2[dir] >> 5), 1u << (r2[dir] & 31u));
+          else if (!((word[dir] >> bit) & 1u)) old[dir] = atomicOr(A.visited + (r2[dir] >> 3), 1u << bit);
+        }
+      }
+#pragma unroll
+      for (int dir = 0; dir < 4; ++dir) {
+        const uint32_t sh = 4 * (r2[dir] & 7u);
+        const bool fresh = !((old[dir] >> (region[dir] > 3 ? r2[dir] & 31u : sh + region[dir])) & 1u);
+        if (fresh) {
+          const uint32_t x = index + (uint32_t)(step[dir] * (int32_t)G::index_weight(j));
+          // the placement's entry is written by its first visit, of any
+          // region; the bits of five regions are in two words, so for these
+          // the entry itself tells (writers of one level write the same value)
+          const bool first = ce[dir].w > 4 ? x != A.goal && __ldcg(A.lookup + x) == 0 : ((old[dir] >> sh) & 15u) == 0;
+          if (first) A.lookup[x] = (uint8_t)(d + 1);
+        }
+        const unsigned got = __ballot_sync(FULL, fresh);
+        if (fresh) buf[n_buf + __popc(got & ((1u << lane) - 1u))] = r2[dir] << 3 | region[dir];
+        n_buf += __popc(got);
+      }
+      __syncwarp();
+      if (n_buf > kBfsBuf - 128) flush();
+      earlier |= 1u << p;
     }
   }
-  if (local) atomicAdd(produced, local);
-}
-
-template <int STRIDE>
-__global__ void region_min_kernel(const uint8_t *dist, uint64_t T, int n, uint8_t *compact) {
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < T;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    const uint8_t *row = dist + r * STRIDE;
-    uint8_t best = kUnseen;
-    for (int m = 0; m < n; ++m) best = min(best, row[m]);
-    compact[r] = best;
+  if (n_buf) flush();
+  // the last block to finish closes the next level
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(A.done, 1u) == gridDim.x - 1) {
+      *A.done = 0;
+      A.bounds[d + 2] = atomicAdd(A.tail, 0u);
+    }
   }
 }
 
-__global__ void compact_lookup_kernel(int n, int k, uint64_t T, const uint8_t *src, uint8_t *dst,
-                                      int to_lookup) {
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < T;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    int pos[6] = {0, 0, 0, 0, 0, 0};
-    unrank_k(n, k, r, pos);
-    const uint32_t x = lookup_index(n, k, pos);
+template <int W>
+__global__ void compact_lookup_kernel(const uint8_t *src, uint8_t *dst, uint32_t T, int to_lookup) {
+  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < T; r += gridDim.x * blockDim.x) {
+    int pos[Geo<W>::K];
+    unrank<W>(r, pos);
+    const uint32_t x = lookup_index<W>(pos);
     if (to_lookup) dst[x] = src[r];
     else dst[r] = src[x];
   }
@@ -214,87 +380,131 @@ uint64_t compact_table_size(int w) {
 
 uint64_t lookup_table_stride(int w) { return w == 4 ? (1ull << 20) : (1ull << 28); }
 
-cudaError_t pdb_compact_to_lookup(int w, int table_id, const uint8_t *compact, uint8_t *lookup,
-                                  cudaStream_t st) {
-  PatternSet ps = pattern_set(w);
+static cudaError_t launch_compact_lookup(int w, const uint8_t *src, uint8_t *dst, int to_lookup, cudaStream_t st) {
   const uint64_t T = compact_table_size(w);
+  if (w == 4) compact_lookup_kernel<4><<<grid_for(T, 256), 256, 0, st>>>(src, dst, (uint32_t)T, to_lookup);
+  else compact_lookup_kernel<5><<<grid_for(T, 256), 256, 0, st>>>(src, dst, (uint32_t)T, to_lookup);
+  note_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t pdb_compact_to_lookup(int w, const uint8_t *compact, uint8_t *lookup, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(lookup, 0, lookup_table_stride(w), st);
   if (e != cudaSuccess) return e;
-  compact_lookup_kernel<<<grid_for(T, 256), 256, 0, st>>>(w * w, ps.k, T, compact, lookup, 1);
-  note_launch();
-  (void)table_id;
-  return cudaGetLastError();
+  return launch_compact_lookup(w, compact, lookup, 1, st);
 }
 
-cudaError_t pdb_lookup_to_compact(int w, int table_id, const uint8_t *lookup, uint8_t *compact,
-                                  cudaStream_t st) {
-  PatternSet ps = pattern_set(w);
-  const uint64_t T = compact_table_size(w);
-  compact_lookup_kernel<<<grid_for(T, 256), 256, 0, st>>>(w * w, ps.k, T, lookup, compact, 0);
-  note_launch();
-  (void)table_id;
-  return cudaGetLastError();
+cudaError_t pdb_lookup_to_compact(int w, const uint8_t *lookup, uint8_t *compact, cudaStream_t st) {
+  return launch_compact_lookup(w, lookup, compact, 0, st);
 }
 
-cudaError_t build_pdb_table(int w, int table_id, uint8_t *lookup, uint8_t *compact,
-                            cudaStream_t st, int *levels_out, double *ms_out) {
-  auto t0 = std::chrono::steady_clock::now();
-  const Geo g = make_geo(w, table_id);
-  const uint64_t T = compact_table_size(w);
-  const int stride = g.n <= 16 ? 16 : 32;
-  uint8_t *dist = nullptr, *cmp = nullptr;
-  unsigned long long *produced = nullptr, *h_produced = nullptr;
-  cudaError_t e = cudaMalloc(&dist, T * (uint64_t)stride);
-  if (e != cudaSuccess) return e;
-  e = cudaMalloc(&cmp, T);
-  if (e == cudaSuccess) e = cudaMalloc(&produced, sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMallocHost(&h_produced, sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemsetAsync(dist, 0xFF, T * (uint64_t)stride, st);
-  if (e == cudaSuccess) {
-    // goal: pattern tiles home, blank in the region of cell 0
-    uint32_t occ = 0;
-    for (int j = 0; j < g.k; ++j) occ |= 1u << g.base[j];
-    const uint32_t reg = flood(g, g.full & ~occ, 0);
-    const uint64_t r0 = rank_k(g.n, g.k, g.base);
-    static const uint8_t zero = 0;
-    e = cudaMemcpyAsync(dist + r0 * stride + (__builtin_ffs((int)reg) - 1), &zero, 1,
-                        cudaMemcpyHostToDevice, st);
+namespace {
+
+// Levels launched between two looks at the queue from the host: the launches
+// after the last level cost about 3 us each, a look about 15.
+constexpr int kLevelsPerLook = 8;
+constexpr int kMaxLevels = 254;  // distances are bytes
+
+// The goal: pattern tiles home, blank in the region of cell 0.
+template <int W>
+Goal goal_state(const PatternSet &ps, int table) {
+  using G = Geo<W>;
+  Goal g{0, 0, 0};
+  uint32_t occ = 0;
+  for (int j = 0; j < G::K; ++j) {
+    const int cell = ps.table_tiles[table][j];
+    g.rank += G::rank_weight(j) * (uint32_t)(cell - __builtin_popcount(occ & ((1u << cell) - 1u)));
+    g.index += G::index_weight(j) * (uint32_t)cell;
+    occ |= 1u << cell;
   }
-  int levels = 0;
-  for (int d = 0; e == cudaSuccess && d < 254; ++d) {
-    e = cudaMemsetAsync(produced, 0, sizeof(unsigned long long), st);
-    if (e != cudaSuccess) break;
-    if (stride == 16)
-      bfs_level_kernel<16><<<grid_for(T, 256), 256, 0, st>>>(dist, T, g, d, produced);
-    else
-      bfs_level_kernel<32><<<grid_for(T, 256), 256, 0, st>>>(dist, T, g, d, produced);
-    note_launch();
-    e = cudaGetLastError();
+  // regions are numbered by their lowest cells, so cell 0's, when it is free
+  // (it is the blank's home), is number 0
+  return g;
+}
+
+template <int W>
+cudaError_t build_tables(uint8_t *lookup, cudaStream_t st) {
+  using G = Geo<W>;
+  const PatternSet ps = pattern_set(W);
+  const uint64_t T = compact_table_size(W);
+  constexpr size_t lo_n = (size_t)1 << G::kLoBits, hi_n = (size_t)1 << (G::N - G::kLoBits);
+  const size_t vis_n = (T + 7) / 8, extra_n = (T + 31) / 32;
+  // one allocation: 16-byte records first, then words; the state counter is 8-byte aligned
+  const size_t words = 4 * (size_t)G::kSubsets + 2 + G::kSubsetWords + lo_n / 2 + hi_n + vis_n + extra_n + kMaxLevels +
+                       kLevelsPerLook + 8;
+  uint32_t *mem = nullptr, *queue = nullptr, *h_bounds = nullptr;
+  cudaError_t e = cudaMalloc(&mem, words * sizeof(uint32_t));
+  if (e == cudaSuccess)
+    e = cudaMallocHost(&h_bounds, (kMaxLevels + kLevelsPerLook + 4) * sizeof(uint32_t));
+  int blocks = 0, dev = 0, sms = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, bfs_level_kernel<W>, kBfsBlock, 0);
+  if (e == cudaSuccess) {
+    BfsArgs A{};
+    A.subsets.regions = reinterpret_cast<uint4 *>(mem);
+    unsigned long long *n_regions = reinterpret_cast<unsigned long long *>(mem + 4 * (size_t)G::kSubsets);
+    A.subsets.split = mem + 4 * (size_t)G::kSubsets + 2;
+    A.subsets.lo = reinterpret_cast<uint16_t *>(A.subsets.split + G::kSubsetWords);
+    A.subsets.hi = A.subsets.split + G::kSubsetWords + lo_n / 2;
+    A.visited = A.subsets.hi + hi_n;
+    A.extra = A.visited + vis_n;
+    A.bounds = A.extra + extra_n;
+    A.tail = A.bounds + kMaxLevels + kLevelsPerLook + 4;
+    A.done = A.tail + 1;
+    // subset tables; the number of states is k! placements for every region of a subset
+    e = cudaMemsetAsync(n_regions, 0, sizeof(unsigned long long) + G::kSubsetWords * sizeof(uint32_t), st);
+    if (e == cudaSuccess) {
+      subset_kernel<W><<<(G::kFull >> 8) + 1, 256, 0, st>>>(A.subsets, n_regions);
+      note_launch();
+      e = cudaGetLastError();
+    }
+    unsigned long long *h_regions = reinterpret_cast<unsigned long long *>(h_bounds);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(h_produced, produced, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+      e = cudaMemcpyAsync(h_regions, n_regions, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    levels = d + 1;
-    if (e != cudaSuccess || *h_produced == 0) break;
+    if (e == cudaSuccess) {
+      uint64_t states = *h_regions;
+      for (int i = 2; i <= G::K; ++i) states *= (uint64_t)i;
+      A.cap = (uint32_t)states;
+      e = cudaMalloc(&queue, states * sizeof(uint32_t));
+      A.queue = queue;
+    }
+    for (int t = 0; e == cudaSuccess && t < ps.n_tables; ++t) {
+      A.lookup = lookup + (size_t)t * lookup_table_stride(W);
+      e = cudaMemsetAsync(A.lookup, 0, lookup_table_stride(W), st);
+      if (e == cudaSuccess) e = cudaMemsetAsync(A.visited, 0, (vis_n + extra_n) * sizeof(uint32_t), st);
+      if (e != cudaSuccess) break;
+      const Goal g = goal_state<W>(ps, t);
+      A.goal = g.index;
+      bfs_start_kernel<<<1, 1, 0, st>>>(A, g);
+      note_launch();
+      e = cudaGetLastError();
+      bool over = false;
+      for (int d = 0; e == cudaSuccess && !over && d < kMaxLevels; d += kLevelsPerLook) {
+        const int n = kMaxLevels - d < kLevelsPerLook ? kMaxLevels - d : kLevelsPerLook;
+        for (int l = 0; l < n && e == cudaSuccess; ++l) {
+          bfs_level_kernel<W><<<sms * blocks, kBfsBlock, 0, st>>>(A, d + l);
+          note_launch();
+          e = cudaGetLastError();
+        }
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(h_bounds, A.bounds + d + n, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        over = e == cudaSuccess && h_bounds[0] == h_bounds[1];
+      }
+    }
   }
-  if (e == cudaSuccess) {
-    if (stride == 16)
-      region_min_kernel<16><<<grid_for(T, 256), 256, 0, st>>>(dist, T, g.n, cmp);
-    else
-      region_min_kernel<32><<<grid_for(T, 256), 256, 0, st>>>(dist, T, g.n, cmp);
-    note_launch();
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = pdb_compact_to_lookup(w, table_id, cmp, lookup, st);
-  if (e == cudaSuccess && compact) e = cudaMemcpyAsync(compact, cmp, T, cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(dist);
-  cudaFree(cmp);
-  cudaFree(produced);
-  cudaFreeHost(h_produced);
-  if (levels_out) *levels_out = levels;
-  if (ms_out)
-    *ms_out = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+  cudaFree(queue);
+  cudaFree(mem);
+  cudaFreeHost(h_bounds);
   return e;
+}
+
+}  // namespace
+
+cudaError_t build_pdb_tables(int w, uint8_t *lookup, cudaStream_t st) {
+  return w == 4 ? build_tables<4>(lookup, st) : build_tables<5>(lookup, st);
 }
 
 cudaError_t launch_heuristic(int w, bool pdb, const uint8_t *boards, int n, int32_t *h,

@@ -232,7 +232,6 @@ struct sp_solver {
   uint8_t *d_pdb = nullptr;
   bool pdb_ready = false;
   uint32_t import_mask = 0;
-  double pdb_build_ms = 0;
   int last_lanes = 0;       // lanes of the last search launch
   uint32_t last_emitted = 0;
   // split pre-pass buffers
@@ -1642,17 +1641,8 @@ int sp_pdb_num_tables(int width) {
 int sp_pdb_build(sp_solver *s) {
   if (!s) return SP_ERR_ARG;
   if (s->heur != SP_HEUR_PDB) return SP_ERR_ARG;
-  const int nt = pattern_set(s->w).n_tables;
-  double total = 0;
-  for (int t = 0; t < nt; ++t) {
-    int levels = 0;
-    double ms = 0;
-    cudaError_t e = build_pdb_table(s->w, t, s->d_pdb + (size_t)t * lookup_table_stride(s->w), nullptr,
-                                    s->st, &levels, &ms);
-    if (e != cudaSuccess) return fail_cuda(s, e, "build_pdb_table");
-    total += ms;
-  }
-  s->pdb_build_ms = total;
+  const cudaError_t e = build_pdb_tables(s->w, s->d_pdb, s->st);
+  if (e != cudaSuccess) return fail_cuda(s, e, "build_pdb_tables");
   s->pdb_ready = true;
   return SP_OK;
 }
@@ -1663,7 +1653,7 @@ int sp_pdb_export(sp_solver *s, int table, uint8_t *dst, uint64_t size) {
   if (!s->pdb_ready) return SP_ERR_NO_PDB;
   uint8_t *tmp = nullptr;
   SP_CUDA(s, cudaMalloc(&tmp, size));
-  cudaError_t e = pdb_lookup_to_compact(s->w, table, s->d_pdb + (size_t)table * lookup_table_stride(s->w), tmp, s->st);
+  cudaError_t e = pdb_lookup_to_compact(s->w, s->d_pdb + (size_t)table * lookup_table_stride(s->w), tmp, s->st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dst, tmp, size, cudaMemcpyDeviceToHost, s->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
   cudaFree(tmp);
@@ -1679,7 +1669,7 @@ int sp_pdb_import(sp_solver *s, int table, const uint8_t *src, uint64_t size) {
   SP_CUDA(s, cudaMalloc(&tmp, size));
   cudaError_t e = cudaMemcpyAsync(tmp, src, size, cudaMemcpyHostToDevice, s->st);
   if (e == cudaSuccess)
-    e = pdb_compact_to_lookup(s->w, table, tmp, s->d_pdb + (size_t)table * lookup_table_stride(s->w), s->st);
+    e = pdb_compact_to_lookup(s->w, tmp, s->d_pdb + (size_t)table * lookup_table_stride(s->w), s->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
   cudaFree(tmp);
   if (e != cudaSuccess) return fail_cuda(s, e, "sp_pdb_import");

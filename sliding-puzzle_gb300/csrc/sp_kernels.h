@@ -144,17 +144,13 @@ cudaError_t launch_frontier(int w, bool pdb, int n_live, const FrontArgs &A, cud
 cudaError_t launch_heuristic(int w, bool pdb, const uint8_t *boards, int n, int32_t *h,
                              const HeurTables *ht, const uint8_t *tables, cudaStream_t st);
 
-// Breadth-first build of table `table_id` of width w into the device lookup
-// layout (mixed radix 16^5 or 25^6 bytes) at `lookup`; also writes the
-// compact rank-order table to `compact` when non-null.  Scratch is allocated
-// and freed inside.
-cudaError_t build_pdb_table(int w, int table_id, uint8_t *lookup, uint8_t *compact,
-                            cudaStream_t st, int *levels_out, double *ms_out);
-// compact rank order <-> lookup layout
-cudaError_t pdb_compact_to_lookup(int w, int table_id, const uint8_t *compact, uint8_t *lookup,
-                                  cudaStream_t st);
-cudaError_t pdb_lookup_to_compact(int w, int table_id, const uint8_t *lookup, uint8_t *compact,
-                                  cudaStream_t st);
+// Breadth-first build of width w's tables into the device lookup layout
+// (mixed radix 16^5 or 25^6 bytes, lookup_table_stride(w) apart).  Scratch
+// (0.8 GB for width 5) is allocated and freed inside.
+cudaError_t build_pdb_tables(int w, uint8_t *lookup, cudaStream_t st);
+// compact rank order <-> lookup layout, one table
+cudaError_t pdb_compact_to_lookup(int w, const uint8_t *compact, uint8_t *lookup, cudaStream_t st);
+cudaError_t pdb_lookup_to_compact(int w, const uint8_t *lookup, uint8_t *compact, cudaStream_t st);
 
 uint64_t compact_table_size(int w);
 uint64_t lookup_table_stride(int w);
