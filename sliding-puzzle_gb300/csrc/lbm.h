@@ -48,7 +48,10 @@ class Model {
   int export_params(float *dst, size_t n, cudaStream_t st, std::string &err);
   bool ready() const { return ready_; }
 
-  // Host arrays: tiles n x N, slack n; out n predictions.
+  // Host arrays: tiles n x N, slack n; out n predictions.  The device checks
+  // the rows (a permutation each, slack 0..255): SP_ERR_NOT_PERMUTATION or
+  // SP_ERR_ARG for the first bad one, out untouched.  train_step likewise:
+  // grads, loss and the model stay as they were.
   int predict(const uint8_t *tiles, const int32_t *slack, int n, float *out, cudaStream_t st,
               std::string &err);
   // Device SubRoots selected by host index lists (idx n, slack n).
@@ -75,7 +78,9 @@ class Model {
 
  private:
   int ensure_batch(int n, std::string &err);
-  int forward_infer(int n, float *out, cudaStream_t st, std::string &err);
+  int forward_infer(int n, size_t off, cudaStream_t st, std::string &err);
+  int predict_rows(const uint8_t *tiles, const SubRoot *d_subs, const uint32_t *idx, const int32_t *slack, int n,
+                   float *out, cudaStream_t st, std::string &err);
 
   int w_;
   bool ready_ = false;

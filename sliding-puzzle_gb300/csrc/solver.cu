@@ -1885,8 +1885,11 @@ int sp_lbm_export(sp_solver *s, float *dst, uint64_t n) {
   return rc ? rc : s->lbm->export_params(dst, (size_t)n, s->st, s->err);
 }
 
+// Argument errors of the model's calls are found in this order: null rows or
+// a negative count, the first bad row, then what else is wrong.  The device
+// checks the rows of a call that has nothing else wrong (lbm.h); this checks
+// them here when something else is.
 static int lbm_check_rows(sp_solver *s, const uint8_t *tiles, const int32_t *slack, int n) {
-  if (!tiles || !slack || n < 0) return SP_ERR_ARG;
   for (int i = 0; i < n; ++i) {
     if (slack[i] < 0 || slack[i] > 255) {
       s->err = "slack must lie in 0..255";
@@ -1907,28 +1910,38 @@ static int lbm_check_rows(sp_solver *s, const uint8_t *tiles, const int32_t *sla
 
 int sp_lbm_predict(sp_solver *s, const uint8_t *tiles, const int32_t *slack, int n, float *out) {
   int rc = lbm_model(s, true);
-  if (!rc) rc = lbm_check_rows(s, tiles, slack, n);
   if (rc) return rc;
-  if (!out) return SP_ERR_ARG;
+  if (!tiles || !slack || n < 0) return SP_ERR_ARG;
+  if (!out) {
+    rc = lbm_check_rows(s, tiles, slack, n);
+    return rc ? rc : SP_ERR_ARG;
+  }
   return n ? s->lbm->predict(tiles, slack, n, out, s->st, s->err) : SP_OK;
+}
+
+// One training call: update with lr, or the gradient alone.
+static int lbm_step(sp_solver *s, const uint8_t *tiles, const int32_t *slack, const float *target, int n, float lr,
+                    bool update, float *loss, float *grads) {
+  int rc = lbm_model(s, true);
+  if (rc) return rc;
+  if (!tiles || !slack || n < 0) return SP_ERR_ARG;
+  const bool args = target && (update ? lr > 0.f : grads != nullptr);
+  if (!args || n <= 0 || n % 128) {  // train_step refuses the size
+    rc = lbm_check_rows(s, tiles, slack, n);
+    if (rc) return rc;
+    if (!args) return SP_ERR_ARG;
+  }
+  return s->lbm->train_step(tiles, slack, target, n, lr, update, loss, grads, s->st, s->err);
 }
 
 int sp_lbm_train_step(sp_solver *s, const uint8_t *tiles, const int32_t *slack, const float *target, int n,
                       float lr, float *loss) {
-  int rc = lbm_model(s, true);
-  if (!rc) rc = lbm_check_rows(s, tiles, slack, n);
-  if (rc) return rc;
-  if (!target || !(lr > 0.f)) return SP_ERR_ARG;
-  return s->lbm->train_step(tiles, slack, target, n, lr, true, loss, nullptr, s->st, s->err);
+  return lbm_step(s, tiles, slack, target, n, lr, true, loss, nullptr);
 }
 
 int sp_lbm_gradients(sp_solver *s, const uint8_t *tiles, const int32_t *slack, const float *target, int n,
                      float *grads, float *loss) {
-  int rc = lbm_model(s, true);
-  if (!rc) rc = lbm_check_rows(s, tiles, slack, n);
-  if (rc) return rc;
-  if (!target || !grads) return SP_ERR_ARG;
-  return s->lbm->train_step(tiles, slack, target, n, 0.f, false, loss, grads, s->st, s->err);
+  return lbm_step(s, tiles, slack, target, n, 0.f, false, loss, grads);
 }
 
 int sp_gemm_bf16_nt(const uint16_t *a, const uint16_t *b, float *c, int m, int n, int k) {
