@@ -2,16 +2,19 @@
 // fused epilogues, Adam.  See lbm.h for the model.
 //
 // GEMM shape: C[M x 256] = A[M x K] . B[256 x K]^T with A and B bf16, K-major
-// (K contiguous), fp32 accumulation in tensor memory.  One CTA of 4 warps
+// (K contiguous), fp32 accumulation in tensor memory.  One CTA of 8 warps
 // computes one 128-row tile over a K range:
 //   * thread 0 streams 64-wide K chunks of A (128 x 64) and B (256 x 64) into
 //     shared memory with TMA (128-byte swizzle), two stages, completion on an
 //     mbarrier, and issues four tcgen05.mma (M=128, N=256, K=16) per chunk;
 //     tcgen05.commit frees a stage once its MMAs have read it;
 //   * warp 0 allocates 256 TMEM columns (the 128 x 256 fp32 accumulator);
-//   * after the last commit all four warps read their 32 accumulator rows
-//     with tcgen05.ld (32x32b) and run the epilogue.
-// The training step is four such GEMMs:
+//   * after the last commit every warp reads half of the columns of its 32
+//     accumulator rows with tcgen05.ld (32x32b) and runs the epilogue.
+// The training step is four such GEMMs in three launches (dZ1 and dW2 do not
+// depend on each other and fill half of the SMs each); with two warps per 32
+// accumulator rows and 16-byte reductions they take 49 us for 8192 24-puzzle
+// rows, 112 before:
 //   forward   Z2 = H1 . W2^T          epilogue: ReLU, layer 3, loss, dL/dy,
 //                                     dH2 = dy w3 (Z2 > 0), d/dw3, d/db2
 //   backward  dZ1 = dH2 . W2          epilogue: dH1 = dZ1 (H1 > 0), d/db1
@@ -49,7 +52,9 @@ constexpr int STAGES = 2;
 constexpr int A_STAGE = BM * BK * 2;         // 16 KB
 constexpr int B_STAGE = H * BK * 2;          // 32 KB
 constexpr int SMEM_TILES = STAGES * (A_STAGE + B_STAGE);
-constexpr int SMEM_BYTES = SMEM_TILES + 1024 /* alignment slack */ + 128 /* barriers, TMEM address */;
+constexpr int SMEM_BYTES = SMEM_TILES + 1024 /* alignment slack */ + 128 /* barriers, TMEM address */ +
+                           2 * BM * 4 /* partial predictions */;
+constexpr int kGemmThreads = 256;            // two warps per 32 accumulator rows, half of the columns each
 // kind::f16 instruction descriptor: D f32 (bits 4-5 = 1), A bf16 (7-9 = 1),
 // B bf16 (10-12 = 1), both K-major (15, 16 = 0), N >> 3 at 17-22, M >> 4 at 24-28
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(H >> 3) << 17) |
@@ -202,10 +207,119 @@ __device__ __forceinline__ void store_bf16x32(__nv_bfloat16 *dst, const float (&
   for (int i = 0; i < 4; ++i) d[i] = make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
 }
 
+// Epilogue of a CTA's 128 x 256 accumulator.  Warp w reads the TMEM lanes
+// 32 * (w & 3) .. of its warpgroup's position, and the columns of half w >> 2.
 template <int EPI>
-__global__ void __launch_bounds__(128, 1)
-    umma_gemm_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int kc_per_cta,
-                     int kc_total, EpiArgs E) {
+__device__ __forceinline__ void epilogue(const EpiArgs &E, uint32_t tmem, int m0, float (*s_y)[BM]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int half = warp >> 2, in_tile = (warp & 3) * 32 + lane;
+  const int row = m0 + in_tile;
+  const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  const bool valid = row < E.m_valid;
+  const int cb = half * (H / 2), ce = cb + H / 2;
+  if (EPI == EPI_F32 || EPI == EPI_F32_ATOMIC) {
+    for (int c0 = cb; c0 < ce; c0 += 32) {
+      float v[32];
+      tmem_ld32(tbase + c0, v);
+      if (valid) {
+        float4 *dst = reinterpret_cast<float4 *>(E.C + (size_t)row * H + c0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 x = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          if (EPI == EPI_F32) dst[j] = x;
+          else atomicAdd(dst + j, x);  // one 16-byte reduction
+        }
+      }
+    }
+  } else if (EPI == EPI_FWD || EPI == EPI_INFER) {
+    float part = 0.f;
+    for (int c0 = cb; c0 < ce; c0 += 32) {
+      float v[32];
+      tmem_ld32(tbase + c0, v);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const float z = v[j] + E.b2[c0 + j];
+        if (z > 0.f) part += z * E.w3[c0 + j];
+      }
+    }
+    s_y[half][in_tile] = part;
+    __syncthreads();
+    const float yv = s_y[0][in_tile] + s_y[1][in_tile] + E.b3[0];
+    if (valid && half == 0) E.y[row] = yv;
+    if (EPI == EPI_FWD) {
+      float dy = 0.f, l = 0.f;
+      if (valid) {
+        const float d = yv - E.target[row];
+        l = d * d;
+        dy = 2.f * d * E.inv_b;
+      }
+      if (half == 0) {
+        l = warp_sum(l);
+        const float sdy = warp_sum(dy);
+        if (lane == 0) {
+          atomicAdd(E.loss, l * E.inv_b);
+          atomicAdd(E.gb3, sdy);
+        }
+      }
+      for (int c0 = cb; c0 < ce; c0 += 32) {
+        float v[32], gw[32], gb[32];
+        tmem_ld32(tbase + c0, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float z = v[j] + E.b2[c0 + j];
+          const float d = z > 0.f ? dy * E.w3[c0 + j] : 0.f;
+          gw[j] = z > 0.f ? dy * z : 0.f;
+          gb[j] = d;
+          v[j] = d;
+        }
+        store_bf16x32(E.dH2 + (size_t)row * H + c0, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) E.dH2T[(size_t)(c0 + j) * E.ldt + row] = __float2bfloat16_rn(v[j]);
+        const float s1 = warp_colsum(gw, lane);
+        const float s2 = warp_colsum(gb, lane);
+        atomicAdd(&E.gw3[c0 + lane], s1);
+        atomicAdd(&E.gb2[c0 + lane], s2);
+      }
+    }
+  } else if (EPI == EPI_BWD1) {
+    for (int c0 = cb; c0 < ce; c0 += 32) {
+      float v[32];
+      tmem_ld32(tbase + c0, v);
+      const uint4 *hp = reinterpret_cast<const uint4 *>(E.H1 + (size_t)row * H + c0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 u = hp[q];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162 *>(&w[e]);
+          const int j = q * 8 + e * 2;
+          if (!(__low2float(h2) > 0.f)) v[j] = 0.f;
+          if (!(__high2float(h2) > 0.f)) v[j + 1] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) E.dH1T[(size_t)(c0 + j) * E.ldt + row] = __float2bfloat16_rn(v[j]);
+      const float s = warp_colsum(v, lane);
+      atomicAdd(&E.gb1[c0 + lane], s);
+    }
+  }
+}
+
+// A GEMM of a launch: its operands, row tiles, and the K chunks of a CTA.
+struct GemmArgs {
+  int m_tiles, kc_per_cta, kc_total;
+  EpiArgs E;
+};
+
+// One launch runs GEMM `a` on its first CTAs and, when EPI2 is given, GEMM
+// `b` on the others: of two that do not depend on each other and fill half of
+// the SMs each.
+template <int EPI, int EPI2>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+    umma_gemm_kernel(const __grid_constant__ CUtensorMap a_a, const __grid_constant__ CUtensorMap a_b,
+                     const __grid_constant__ GemmArgs a, const __grid_constant__ CUtensorMap b_a,
+                     const __grid_constant__ CUtensorMap b_b, const __grid_constant__ GemmArgs b, int ctas_a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t *sA = smem;
@@ -213,10 +327,16 @@ __global__ void __launch_bounds__(128, 1)
   uint64_t *bars = (uint64_t *)(smem + SMEM_TILES);  // full[2], done[2], accum
   uint32_t *tmem_holder = (uint32_t *)(bars + 6);
   int *s_fail = (int *)(bars + 7);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM;
-  const int kc0 = blockIdx.y * kc_per_cta;
-  const int nk = min(kc_per_cta, kc_total - kc0);
+  float(*s_y)[BM] = reinterpret_cast<float(*)[BM]>(smem + SMEM_TILES + 128);
+  const int warp = threadIdx.x >> 5;
+  const bool second = EPI2 >= 0 && (int)blockIdx.x >= ctas_a;
+  const CUtensorMap *ta = second ? &b_a : &a_a, *tb = second ? &b_b : &a_b;
+  const GemmArgs &G = second ? b : a;
+  const EpiArgs &E = G.E;
+  const int cta = (int)blockIdx.x - (second ? ctas_a : 0);
+  const int m0 = (cta % G.m_tiles) * BM;
+  const int kc0 = (cta / G.m_tiles) * G.kc_per_cta;
+  const int nk = min(G.kc_per_cta, G.kc_total - kc0);
   const uint32_t full0 = smem_u32(bars), done0 = smem_u32(bars + 2), accum = smem_u32(bars + 4);
 
   if (threadIdx.x == 0) {
@@ -241,8 +361,8 @@ __global__ void __launch_bounds__(128, 1)
       const int s = kc % STAGES;
       if (kc0 + kc + 1 != E.starve_kc1) {
         mbar_expect_tx(full0 + 8 * s, A_STAGE + B_STAGE);
-        tma_load_2d(&ta, smem_u32(sA + s * A_STAGE), full0 + 8 * s, (kc0 + kc) * BK, m0);
-        tma_load_2d(&tb, smem_u32(sB + s * B_STAGE), full0 + 8 * s, (kc0 + kc) * BK, 0);
+        tma_load_2d(ta, smem_u32(sA + s * A_STAGE), full0 + 8 * s, (kc0 + kc) * BK, m0);
+        tma_load_2d(tb, smem_u32(sB + s * B_STAGE), full0 + 8 * s, (kc0 + kc) * BK, 0);
       }
       ++issued;
     };
@@ -280,96 +400,14 @@ __global__ void __launch_bounds__(128, 1)
     umma_commit(accum);  // arrives once every MMA issued above has completed
   }
   __syncthreads();
-  const bool have = mbar_wait(accum, 0, limit) && !*(volatile int *)s_fail;
+  // the same answer for all threads: the epilogue has a barrier
+  const bool have = __syncthreads_and(mbar_wait(accum, 0, limit) && !*(volatile int *)s_fail);
   if (!have && E.err) atomicExch(E.err, 1);
   tc_fence_after();
 
   if (have) {
-    const int row = m0 + warp * 32 + lane;
-    const uint32_t tbase = tmem + ((uint32_t)(warp * 32) << 16);
-    const bool valid = row < E.m_valid;
-    if (EPI == EPI_F32 || EPI == EPI_F32_ATOMIC) {
-      for (int c0 = 0; c0 < H; c0 += 32) {
-        float v[32];
-        tmem_ld32(tbase + c0, v);
-        if (valid) {
-          float *dst = E.C + (size_t)row * H + c0;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (EPI == EPI_F32) dst[j] = v[j];
-            else atomicAdd(dst + j, v[j]);
-          }
-        }
-      }
-    } else if (EPI == EPI_FWD || EPI == EPI_INFER) {
-      float yv = 0.f;
-      for (int c0 = 0; c0 < H; c0 += 32) {
-        float v[32];
-        tmem_ld32(tbase + c0, v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const float z = v[j] + E.b2[c0 + j];
-          if (z > 0.f) yv += z * E.w3[c0 + j];
-        }
-      }
-      yv += E.b3[0];
-      if (valid) E.y[row] = yv;
-      if (EPI == EPI_FWD) {
-        float dy = 0.f, l = 0.f;
-        if (valid) {
-          const float d = yv - E.target[row];
-          l = d * d;
-          dy = 2.f * d * E.inv_b;
-        }
-        l = warp_sum(l);
-        const float sdy = warp_sum(dy);
-        if (lane == 0) {
-          atomicAdd(E.loss, l * E.inv_b);
-          atomicAdd(E.gb3, sdy);
-        }
-        for (int c0 = 0; c0 < H; c0 += 32) {
-          float v[32], gw[32], gb[32];
-          tmem_ld32(tbase + c0, v);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float z = v[j] + E.b2[c0 + j];
-            const float d = z > 0.f ? dy * E.w3[c0 + j] : 0.f;
-            gw[j] = z > 0.f ? dy * z : 0.f;
-            gb[j] = d;
-            v[j] = d;
-          }
-          store_bf16x32(E.dH2 + (size_t)row * H + c0, v);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) E.dH2T[(size_t)(c0 + j) * E.ldt + row] = __float2bfloat16_rn(v[j]);
-          const float s1 = warp_colsum(gw, lane);
-          const float s2 = warp_colsum(gb, lane);
-          atomicAdd(&E.gw3[c0 + lane], s1);
-          atomicAdd(&E.gb2[c0 + lane], s2);
-        }
-      }
-    } else if (EPI == EPI_BWD1) {
-      for (int c0 = 0; c0 < H; c0 += 32) {
-        float v[32];
-        tmem_ld32(tbase + c0, v);
-        const uint4 *hp = reinterpret_cast<const uint4 *>(E.H1 + (size_t)row * H + c0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint4 u = hp[q];
-          const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162 *>(&w[e]);
-            const int j = q * 8 + e * 2;
-            if (!(__low2float(h2) > 0.f)) v[j] = 0.f;
-            if (!(__high2float(h2) > 0.f)) v[j + 1] = 0.f;
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 32; ++j) E.dH1T[(size_t)(c0 + j) * E.ldt + row] = __float2bfloat16_rn(v[j]);
-        const float s = warp_colsum(v, lane);
-        atomicAdd(&E.gb1[c0 + lane], s);
-      }
-    }
+    if (second) epilogue<EPI2 < 0 ? EPI : EPI2>(E, tmem, m0, s_y);
+    else epilogue<EPI>(E, tmem, m0, s_y);
   }
   tc_fence_before();
   __syncthreads();
@@ -583,22 +621,42 @@ int make_map(CUtensorMap *m, const void *ptr, uint64_t rows, uint64_t k, uint32_
   return SP_OK;
 }
 
+// A GEMM and, on the rest of the SMs, another one (m_tiles 0: none).
+struct GemmCall {
+  CUtensorMap ta, tb;
+  int m_tiles = 0, kc_total = 0, splits = 1;
+  EpiArgs E{};
+};
+template <int EPI, int EPI2>
+cudaError_t launch_gemms(const GemmCall &x, const GemmCall &y, cudaStream_t st) {
+  // per device context: the attribute is cheap to set and is not cached
+  cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<EPI, EPI2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       SMEM_BYTES);
+  if (e != cudaSuccess) return e;
+  auto args = [](const GemmCall &c, int &ctas) {
+    const int splits = std::max(1, std::min(c.splits, c.kc_total));
+    const int per = std::max(1, (c.kc_total + splits - 1) / splits);
+    ctas = c.m_tiles * ((c.kc_total + per - 1) / per);  // every CTA gets at least one chunk
+    return GemmArgs{std::max(1, c.m_tiles), per, c.kc_total, c.E};
+  };
+  int na = 0, nb = 0;
+  const GemmArgs a = args(x, na), b = args(y, nb);
+  if (EPI2 < 0) nb = 0;
+  umma_gemm_kernel<EPI, EPI2><<<na + nb, kGemmThreads, SMEM_BYTES, st>>>(x.ta, x.tb, a, y.ta, y.tb, b, na);
+  note_launch(1);
+  return cudaGetLastError();
+}
 template <int EPI>
 cudaError_t launch_gemm(const CUtensorMap &ta, const CUtensorMap &tb, int m_tiles, int kc_total, int splits,
                         const EpiArgs &E, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  splits = std::max(1, std::min(splits, kc_total));
-  const int per = (kc_total + splits - 1) / splits;
-  splits = (kc_total + per - 1) / per;  // every CTA gets at least one chunk
-  umma_gemm_kernel<EPI><<<dim3(m_tiles, splits), 128, SMEM_BYTES, st>>>(ta, tb, per, kc_total, E);
-  note_launch(1);
-  return cudaGetLastError();
+  GemmCall c;
+  c.ta = ta;
+  c.tb = tb;
+  c.m_tiles = m_tiles;
+  c.kc_total = kc_total;
+  c.splits = splits;
+  c.E = E;
+  return launch_gemms<EPI, -1>(c, c, st);
 }
 
 uint64_t splitmix(uint64_t &x) {
@@ -640,6 +698,11 @@ struct Buffers {
   }
 };
 constexpr size_t kFlagWords = 3;  // scal, err, bad
+// CTAs over which the weight gradients' K (the batch) is split: each adds its
+// 128 x 256 partial sum with 16-byte reductions.  8192 rows, two weight
+// gradients: 150 CTAs and scalar atomics 70 us; 100 CTAs 27 us, 32 and 150
+// the same within 5 % (32000 rows: 32 CTAs 15 % slower).
+constexpr int kSplitCtas = 100;
 
 // The status of a call whose rows had a bad one.
 static int bad_row(uint32_t key, std::string &err) {
@@ -938,21 +1001,27 @@ int Model::train_step(const uint8_t *tiles, const int32_t *slack, const float *t
   E.m_valid = n;
   if ((rc = make_map(&m_a, B.H1, n, H, BM, err)) || (rc = make_map(&m_b, B.W2b, H, H, H, err))) return rc;
   LBM_CUDA(launch_gemm<EPI_FWD>(m_a, m_b, n / BM, H / BK, 1, E, st));
-  // dZ1 = dH2 . W2
-  if ((rc = make_map(&m_a, B.dH2, n, H, BM, err)) || (rc = make_map(&m_b, B.W2Tb, H, H, H, err))) return rc;
-  LBM_CUDA(launch_gemm<EPI_BWD1>(m_a, m_b, n / BM, H / BK, 1, E, st));
-  // dW2 = dH2^T . H1 (K = batch, split over about 150 CTAs)
+  // dZ1 = dH2 . W2 and, beside it, dW2 = dH2^T . H1 (K = the batch, split)
   const int kc = n / BK;
-  E.C = B.G + B.oW2;
-  E.m_valid = H;
-  if ((rc = make_map(&m_a, B.dH2T, H, n, BM, err)) || (rc = make_map(&m_b, B.H1T, H, n, H, err))) return rc;
-  LBM_CUDA(launch_gemm<EPI_F32_ATOMIC>(m_a, m_b, H / BM, kc, 75, E, st));
+  GemmCall dz, dw;
+  dz.m_tiles = n / BM;
+  dz.kc_total = H / BK;
+  dz.E = E;
+  if ((rc = make_map(&dz.ta, B.dH2, n, H, BM, err)) || (rc = make_map(&dz.tb, B.W2Tb, H, H, H, err))) return rc;
+  dw.m_tiles = H / BM;
+  dw.kc_total = kc;
+  dw.splits = kSplitCtas / dw.m_tiles;
+  dw.E = E;
+  dw.E.C = B.G + B.oW2;
+  dw.E.m_valid = H;
+  if ((rc = make_map(&dw.ta, B.dH2T, H, n, BM, err)) || (rc = make_map(&dw.tb, B.H1T, H, n, H, err))) return rc;
+  LBM_CUDA((launch_gemms<EPI_BWD1, EPI_F32_ATOMIC>(dz, dw, st)));
   // dW1 = X^T . dH1
   E.C = B.G + B.oW1;
   E.m_valid = B.D;
   if ((rc = make_map(&m_a, B.XT, B.Dpad, n, BM, err)) || (rc = make_map(&m_b, B.dH1T, H, n, H, err))) return rc;
-  LBM_CUDA(launch_gemm<EPI_F32_ATOMIC>(m_a, m_b, B.Dpad / BM, kc, std::max(1, 150 / (B.Dpad / BM)), E, st));
-  launches_ += 5;
+  LBM_CUDA(launch_gemm<EPI_F32_ATOMIC>(m_a, m_b, B.Dpad / BM, kc, std::max(1, kSplitCtas / (B.Dpad / BM)), E, st));
+  launches_ += 4;
   if (update) {
     ++adam_t_;
     const float c1 = 1.f - std::pow(0.9f, (float)adam_t_), c2 = 1.f - std::pow(0.999f, (float)adam_t_);
