@@ -134,43 +134,36 @@ __device__ __forceinline__ uint32_t first_move(uint32_t mask) { return (0x121312
 #define SP_MULTI_PIECE 1.0
 #endif
 
-// Iteration r of instance i, published beside the one before it (warp
-// advance below): its limit and solution record (those of r - 2, whose goal
-// flag is clear), loads zeroed, its na roots (in maxf order, unsplit) at
-// pool indices t0 ... t0 + na - 1, already reserved.  Kept out of line so
-// that the search loop's registers do not pay for it.
-__device__ __noinline__ void publish_second(const RoundParams &P, uint32_t i, int r, int L, uint32_t base,
-                                            uint32_t ns, uint32_t t0, uint32_t na) {
-  const int lane = threadIdx.x & 31;
-  PoolCtl *ctl = P.ctl;
-  if (lane == 0) {
-    const_cast<int32_t *>(P.inst_limit)[2 * i + (r & 1)] = L;
-    P.inst_pair[i] = 1u;
+// Multi-iteration mode: an iteration's roots go out as bulk tasks, each for
+// up to kBulk of them: Task::sub is the first one's place (in P.order when
+// `mask` is not 0, else the SubRoot itself), `plen` their number, bit 7 of
+// `flags` set.  The warp whose lane claims a bulk publishes its roots, one per
+// lane, so that the advancing warp's own publication takes a few rounds
+// instead of one per 32 roots, each with a slot's acquire and release behind
+// it.  Bulks are not counted as outstanding: their roots are, from the start.
+constexpr uint32_t kBulk = 32;
+constexpr uint32_t kBulkFlag = 0x80u;
+
+// Publish task `D` at reserved pool index t (multi-iteration mode, where every
+// index must be filled): waits a bounded time for the slot.
+__device__ __forceinline__ void publish_root(const RoundParams &P, uint32_t t, uint32_t sub, uint32_t plen,
+                                             uint32_t mask, uint32_t flags) {
+  const uint32_t s = t & (P.cap - 1u);
+  bool free_slot = false;
+  for (int spin = 0; spin < (1 << 14) && !free_slot; ++spin) {
+    free_slot = ld_acquire(&P.seq[s]) == t;
+    if (!free_slot) __nanosleep(64);
   }
-  unsigned long long *lz = P.sub_loads + (size_t)(r & 1) * P.n_subs + base;
-  for (uint32_t q = lane; q < ns; q += 32) lz[q] = 0;
-  __threadfence();
-  __syncwarp();
-  const uint32_t mask = P.cap - 1u;
-  for (uint32_t q = lane; q < na; q += 32) {
-    const uint32_t t = t0 + q;
-    bool free_slot = false;
-    for (int spin = 0; spin < (1 << 14) && !free_slot; ++spin) {
-      free_slot = ld_acquire(&P.seq[t & mask]) == t;
-      if (!free_slot) __nanosleep(64);
-    }
-    if (!free_slot) {
-      if (atomicCAS(&ctl->error, 0, SP_ERR_CAPACITY) == 0) ctl->err_info[0] = t;
-      continue;
-    }
-    Task *D = &P.tasks[t & mask];
-    D->sub = base + q;
-    D->plen = 0;
-    D->mask = 0xF;
-    D->flags = (uint8_t)((r & 1) << 6);
-    st_release(&P.seq[t & mask], t + 1u);
+  if (!free_slot) {
+    if (atomicCAS(&P.ctl->error, 0, SP_ERR_CAPACITY) == 0) P.ctl->err_info[0] = t;
+    return;
   }
-  __syncwarp();
+  Task *D = &P.tasks[s];
+  D->sub = sub;
+  D->plen = (uint16_t)plen;
+  D->mask = (uint8_t)mask;
+  D->flags = (uint8_t)flags;
+  st_release(&P.seq[s], t + 1u);
 }
 
 // Multi-iteration mode: the warp of the lane that finished an instance's last
@@ -183,30 +176,57 @@ __device__ __noinline__ void publish_second(const RoundParams &P, uint32_t i, in
 // would crowd the search loop.  When the instance's next iteration is
 // predicted small (below P.pair_nodes) it is published together with this
 // one, and the call that completes such a pair settles both in order.
+// Bound by latency: nothing of the instance runs meanwhile.  So the reads of
+// its state are in flight together, the searches for the active roots take 32
+// probes at a time, the two passes over the roots' loads (sum and histogram;
+// order and split) have eight loads in flight, all arithmetic is 32-bit float
+// (it only orders and splits work), and the publication goes out in bulks.
+// The device loop's launch on 100 random 15-puzzles 3.2 -> 2.6 ms, on one
+// 15-puzzle walk of 40 moves 0.61 -> 0.52 ms.
 __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint32_t *hist) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   PoolCtl *ctl = P.ctl;
-  auto interior = [&](int L) -> unsigned long long {
-    const uint32_t off = P.inter_off[i];
-    int lo = 0, hi = (int)P.inter_len[i];  // first entry with f > L
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (P.inter_f[off + mid] <= L) lo = mid + 1;
-      else hi = mid;
-    }
-    return lo ? P.inter_cum[off + lo - 1] : 0ull;
-  };
   // per instance, two limits and two solution records, by iteration parity
   int r = ld_volatile(&P.inst_iter[i]);
-  int L = ld_volatile(&P.inst_limit[2 * i + (r & 1)]);
-  if (lane == 0) atomicAdd(&P.iter_nodes[(size_t)i * kMaxIters + r], interior(L));
-  if (ld_volatile(&P.inst_pair[i])) {
+  const uint32_t pair = ld_volatile(&P.inst_pair[i]);
+  const int lim0 = ld_volatile(&P.inst_limit[2 * i]), lim1 = ld_volatile(&P.inst_limit[2 * i + 1]);
+  const uint32_t flag0 = ld_volatile(&P.sol[2 * i].flag), flag1 = ld_volatile(&P.sol[2 * i + 1].flag);
+  const int goal = P.goal_maxf[i];
+  const uint32_t base = P.inst_sub_base[i], ns = P.inst_nsub[i];
+  const uint32_t ioff = P.inter_off[i], ilen = P.inter_len[i];
+  // children of root-set interior nodes within L (entries ascending in f)
+  auto interior = [&](int L) -> unsigned long long {
+    uint32_t n = 0;
+    for (uint32_t q = 0; q < ilen; q += 32) {
+      const unsigned in = __ballot_sync(FULL, q + lane < ilen && P.inter_f[ioff + q + lane] <= L);
+      n += (uint32_t)__popc(in);
+      if (in != FULL) break;
+    }
+    return n ? P.inter_cum[ioff + n - 1] : 0ull;
+  };
+  // number of active roots: the prefix of [lo, ns) with maxf <= L, 32 probes a step
+  auto active = [&](uint32_t lo, int L) -> uint32_t {
+    uint32_t hi = ns;  // roots below lo are active, roots from hi on are not
+    while (lo < hi) {
+      const uint32_t step = (hi - lo + 31) / 32, at = lo + (uint32_t)lane * step;
+      const unsigned in = __ballot_sync(FULL, at < hi && P.sub_maxf[base + at] <= L);
+      if (!in) break;  // root lo is not active
+      const uint32_t last = lo + (31u - (uint32_t)__clz(in)) * step;  // active
+      hi = min(hi, last + step);
+      lo = last + 1;
+    }
+    return lo;
+  };
+  int L = r & 1 ? lim1 : lim0;
+  {
+    const unsigned long long in = interior(L);
+    if (lane == 0) atomicAdd(&P.iter_nodes[(size_t)i * kMaxIters + r], in);
+  }
+  if (pair) {
     // iterations r and r + 1 ran together and have both finished: r's goal
     // decides first (r + 1's counts are then never read)
-    int stop = 0;
-    if (lane == 0) stop = (ld_volatile(&P.sol[2 * i + (r & 1)].flag) != 0u || P.goal_maxf[i] <= L) ? 1 : 0;
-    stop = __shfl_sync(FULL, stop, 0);
+    const bool stop = (r & 1 ? flag1 : flag0) != 0u || goal <= L;
     if (stop || r + 1 >= kMaxIters) {
       if (lane == 0) {
         P.inst_final[i] = r;
@@ -217,17 +237,16 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
     }
     ++r;
     L += 2;
+    const unsigned long long in = interior(L);
     if (lane == 0) {
       P.inst_iter[i] = r;
       P.inst_pair[i] = 0u;
-      atomicAdd(&P.iter_nodes[(size_t)i * kMaxIters + r], interior(L));
+      atomicAdd(&P.iter_nodes[(size_t)i * kMaxIters + r], in);
     }
   }
   for (;;) {
     // every task of iteration r has finished: the goal flag is final
-    int stop = 0;
-    if (lane == 0) stop = (ld_volatile(&P.sol[2 * i + (r & 1)].flag) != 0u || P.goal_maxf[i] <= L) ? 1 : 0;
-    stop = __shfl_sync(FULL, stop, 0);
+    const bool stop = (r & 1 ? flag1 : flag0) != 0u || goal <= L;
     if (stop || r + 1 >= kMaxIters) {
       if (lane == 0) {
         P.inst_final[i] = r;
@@ -238,33 +257,65 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
     }
     ++r;
     L += 2;
-    const uint32_t base = P.inst_sub_base[i], ns = P.inst_nsub[i];
-    uint32_t lo = 0, hi = ns;  // active roots: prefix with maxf <= L
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (P.sub_maxf[base + mid] <= L) lo = mid + 1;
-      else hi = mid;
-    }
-    const uint32_t na = lo;
+    const uint32_t na = active(0, L);
     if (lane == 0) {
       P.inst_iter[i] = r;
       const_cast<int32_t *>(P.inst_limit)[2 * i + (r & 1)] = L;
-      if (!na) atomicAdd(&P.iter_nodes[(size_t)i * kMaxIters + r], interior(L));
     }
-    if (!na) continue;
-    // loads of iteration r - 1 (summed by atomics in L2: read past L1)
+    if (!na) {
+      const unsigned long long in = interior(L);
+      if (lane == 0) atomicAdd(&P.iter_nodes[(size_t)i * kMaxIters + r], in);
+      continue;
+    }
+    // loads of iteration r - 1 (summed by atomics in L2: read past L1); the
+    // prediction of root q's next load is that times the root's own predicted
+    // growth (learned balancer; otherwise the instance's, common to all)
     const unsigned long long *ld = P.sub_loads + (size_t)((r - 1) & 1) * P.n_subs + base;
     unsigned long long *nx = P.sub_loads + (size_t)(r & 1) * P.n_subs + base;
+    auto pred_load = [&](uint32_t q, unsigned long long load) -> float {
+      float lq = (float)load;
+      if (P.sub_growth && load) {
+        const int j = min(kGrowthSlacks - 1, max(0, (L - 2 - P.sub_maxf[base + q]) >> 1));
+        lq *= exp2f((float)P.sub_growth[(size_t)(base + q) * kGrowthSlacks + j] * (1.0f / 16.0f));
+      }
+      return lq;
+    };
+    // longest first: bucket = binary exponent of the prediction (0: no load)
+    auto bucket = [](float lq) -> int {
+      return lq >= 1.0f ? min(31, (int)((__float_as_uint(lq) >> 23) & 0xFFu) - 126) : 0;
+    };
+    hist[lane] = 0;
+    __syncwarp();
     unsigned long long tot = 0;
-    for (uint32_t q = lane; q < na; q += 32) tot += __ldcg(ld + q);
-    for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(FULL, tot, o);
+    float ptot = 0.f;
+    for (uint32_t q0 = 0; q0 < na; q0 += 256) {
+      unsigned long long v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t q = q0 + 32 * u + lane;
+        v[u] = q < na ? __ldcg(ld + q) : 0ull;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t q = q0 + 32 * u + lane;
+        if (q >= na) continue;
+        tot += v[u];
+        const float lq = pred_load(q, v[u]);
+        ptot += lq;
+        atomicAdd(&hist[bucket(lq)], 1u);
+      }
+    }
+    for (int o = 16; o; o >>= 1) {
+      tot += __shfl_xor_sync(FULL, tot, o);
+      ptot += __shfl_xor_sync(FULL, ptot, o);
+    }
     // the next iteration's size: this one's times the instance's growth
-    double grow = 6.0;
+    float grow = 6.0f;
     if (r >= 2) {
       const unsigned long long prev = __ldcg(&P.iter_nodes[(size_t)i * kMaxIters + (r - 2)]);
-      if (prev) grow = fmin(30.0, fmax(2.0, (double)tot / (double)prev));
+      if (prev) grow = fminf(30.0f, fmaxf(2.0f, (float)tot / (float)prev));
     }
-    if (P.handback_nodes && (double)tot * grow >= (double)P.handback_nodes) {
+    if (P.handback_nodes && (float)tot * grow >= (float)P.handback_nodes) {
       // a large iteration is next: the host round loop finishes this
       // instance (its loads of iteration r - 1 stay in `ld`)
       if (lane == 0) {
@@ -274,35 +325,8 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
       }
       return;
     }
-    // next-iteration load of root q: its load times its predicted growth
-    // (learned balancer; otherwise the load itself, the instance's growth
-    // being common to all its roots)
-    auto pred_load = [&](uint32_t q) -> double {
-      double lq = (double)__ldcg(ld + q);
-      if (P.sub_growth && lq > 0.0) {
-        const int j = min(kGrowthSlacks - 1, max(0, (L - 2 - P.sub_maxf[base + q]) >> 1));
-        lq *= exp2((double)P.sub_growth[(size_t)(base + q) * kGrowthSlacks + j] * (1.0 / 16.0));
-      }
-      return lq;
-    };
-    double ptot = (double)tot;
-    if (P.sub_growth) {
-      ptot = 0.0;
-      for (uint32_t q = lane; q < na; q += 32) ptot += pred_load(q);
-      for (int o = 16; o; o >>= 1) ptot += __shfl_xor_sync(FULL, ptot, o);
-    }
-    const double avg = ptot / (double)na;
+    const float avg = ptot / (float)na;
     for (uint32_t q = lane; q < ns; q += 32) nx[q] = 0;
-    // longest first: bucket = binary exponent of load / average (0 = no load)
-    auto bucket = [&](double lq) -> int {
-      if (!(lq > 0.0) || !(avg > 0.0)) return 0;
-      int e = 0;
-      frexp(lq / avg, &e);
-      return min(31, max(1, e + 15));
-    };
-    hist[lane] = 0;
-    __syncwarp();
-    for (uint32_t q = lane; q < na; q += 32) atomicAdd(&hist[bucket(pred_load(q))], 1u);
     __syncwarp();
     const uint32_t c = hist[lane];
     uint32_t suf = c;  // roots in buckets >= lane
@@ -311,73 +335,83 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
       if (lane + o < 32) suf += v;
     }
     hist[lane] = suf - c;  // first position of bucket `lane`
+    __syncwarp();
     // iteration r + 1 goes out with r when it is predicted small: the two
     // run together and the instance advances once both have finished, so a
     // chain of small iterations is not paced by one iteration at a time
     uint32_t na2 = 0;
-    if (P.pair_nodes && r + 2 < kMaxIters && (double)tot * grow * grow < (double)P.pair_nodes) {
-      uint32_t lo2 = na, hi2 = ns;  // active roots of r + 1: prefix with maxf <= L + 2
-      while (lo2 < hi2) {
-        const uint32_t mid = (lo2 + hi2) >> 1;
-        if (P.sub_maxf[base + mid] <= L + 2) lo2 = mid + 1;
-        else hi2 = mid;
+    if (P.pair_nodes && r + 2 < kMaxIters && (float)tot * grow * grow < (float)P.pair_nodes) na2 = active(na, L + 2);
+    // the roots in order, each with its split: root q | levels << 26
+    const float piece = avg * (float)SP_MULTI_PIECE;
+    for (uint32_t q0 = 0; q0 < na; q0 += 256) {
+      unsigned long long v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t q = q0 + 32 * u + lane;
+        v[u] = q < na ? __ldcg(ld + q) : 0ull;
       }
-      na2 = lo2;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const uint32_t q = q0 + 32 * u + lane;
+        if (q >= na) continue;
+        const float lq = pred_load(q, v[u]);
+        const uint32_t at = atomicAdd(&hist[bucket(lq)], 1u);
+        int kk = 0;
+        if (P.static_split && piece > 0.f && lq > 2.0f * piece) {
+          // static split from the loads just measured: a root with x pieces'
+          // load goes out as a split task of about log(x)/log(2.4) levels (the
+          // reference cuts it into ceil(load/avg) pieces,
+          // src/24puzzle_block_parallel_with_pdb.cu:839-897)
+          kk = (int)ceilf(__log2f(lq / piece) * (1.0f / 1.2630344f));
+          kk = max(0, min(kk, min(10, L - (int)P.subs[base + q].g - 1)));
+        }
+        P.order[base + at] = q | (uint32_t)kk << 26;
+      }
     }
+    if (na2) {
+      unsigned long long *lz = P.sub_loads + (size_t)((r + 1) & 1) * P.n_subs + base;
+      for (uint32_t q = lane; q < ns; q += 32) lz[q] = 0;
+      if (lane == 0) {
+        const_cast<int32_t *>(P.inst_limit)[2 * i + ((r + 1) & 1)] = L + 2;
+        P.inst_pair[i] = 1u;
+      }
+    }
+    __threadfence();
+    __syncwarp();
     // the whole iteration (pair) is outstanding before its first task is visible
+    const uint32_t nb = (na + kBulk - 1) / kBulk, nb2 = (na2 + kBulk - 1) / kBulk;
     uint32_t t0 = 0;
     if (lane == 0) {
       atomicAdd(&P.inst_out[i], na + na2);
       atomicAdd(&ctl->outstanding, na + na2);
-      t0 = atomicAdd(&ctl->tail, na + na2);
       __threadfence();
+      t0 = atomicAdd(&ctl->tail, nb + nb2);
     }
     t0 = __shfl_sync(FULL, t0, 0);
-    __syncwarp();
-    const uint32_t mask = P.cap - 1u;
-    for (uint32_t q = lane; q < na; q += 32) {
-      const double lq = pred_load(q);
-      const uint32_t t = t0 + atomicAdd(&hist[bucket(lq)], 1u);
-      int kk = 0;
-      const double piece = avg * SP_MULTI_PIECE;
-      if (P.static_split && piece > 0 && lq > 2.0 * piece) {
-        // static split from the loads just measured: a root with x pieces'
-        // load goes out as a split task of about log(x)/log(2.4) levels (the
-        // reference cuts it into ceil(load/avg) pieces,
-        // src/24puzzle_block_parallel_with_pdb.cu:839-897)
-        kk = (int)ceil(log(lq / piece) / log(2.4));
-        kk = max(0, min(kk, min(10, L - (int)P.subs[base + q].g - 1)));
-      }
-      bool free_slot = false;
-      for (int spin = 0; spin < (1 << 14) && !free_slot; ++spin) {
-        free_slot = ld_acquire(&P.seq[t & mask]) == t;
-        if (!free_slot) __nanosleep(64);
-      }
-      if (!free_slot) {
-        if (atomicCAS(&ctl->error, 0, SP_ERR_CAPACITY) == 0) ctl->err_info[0] = t;
-        continue;
-      }
-      Task *D = &P.tasks[t & mask];
-      D->sub = base + q;
-      D->plen = 0;
-      D->mask = 0xF;
-      D->flags = (uint8_t)(kk | ((r & 1) << 6));  // bit 6: the iteration's parity
-      st_release(&P.seq[t & mask], t + 1u);
+    for (uint32_t b = lane; b < nb + nb2; b += 32) {
+      const bool second = b >= nb;
+      const uint32_t q0 = (second ? b - nb : b) * kBulk, left = (second ? na2 : na) - q0;
+      publish_root(P, t0 + b, base + q0, min(kBulk, left), second ? 0u : 1u,
+                   kBulkFlag | (uint32_t)((second ? r + 1 : r) & 1) << 6);
     }
     __syncwarp();
-    if (na2) publish_second(P, i, r + 1, L + 2, base, ns, t0 + na, na2);
     return;
   }
 }
 
-// Most lanes of a warp that donate in one pass of its loop.
+// Most lanes of a warp that donate in one pass of its loop (4 / 8 / 16: one
+// random 15-puzzle 2.87 / 2.64 / 2.57 ms, 100 of them 19.2 / 18.8 / 18.9).
 #ifndef SP_MAX_DONORS
-#define SP_MAX_DONORS 8
+#define SP_MAX_DONORS 16
 #endif
 
-// Longest sleep of a warp with no lane searching between pool polls (ns).
+// Longest sleep of a warp with no lane searching between pool polls (ns): a
+// new iteration waits for it, other warps lose issue slots to the polls (512 /
+// 2048 / 4096 / 16384: one random 15-puzzle 3.4 / 2.8 / 2.65 / 2.76 ms, 50
+// 24-puzzles 19.8 / 19.2 / 19.2 / 20.0, a walk of 40 moves 0.89 / 0.72 / 0.70 /
+// 0.84).
 #ifndef SP_MAX_BACKOFF_NS
-#define SP_MAX_BACKOFF_NS 16384
+#define SP_MAX_BACKOFF_NS 4096
 #endif
 
 // Resident threads per SM that the search kernels are compiled for, and the
@@ -540,7 +574,9 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
   //  * kDebt: a reserved pool index (s_cold1) whose ring slot did not free
   //    in time is owed: the lane kept the work and publishes a null task (no
   //    moves, SubRoot s_cold2) there later, so no index stays unpublished.
-  constexpr uint32_t kAdvance = 1u, kDebt = 2u;
+  //  * kBulkHeld: the lane claimed a bulk (its first place and its header in
+  //    the lane's words for a task's SubRoot and split).
+  constexpr uint32_t kAdvance = 1u, kDebt = 2u, kBulkHeld = 4u;
   uint32_t events = 0;
 
   auto board_off = [&](int c) -> uint32_t {
@@ -690,6 +726,13 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     const Task *T = &P.tasks[s];
     sub = __ldcg(&T->sub);
     const uint32_t hdr = __ldcg((const uint32_t *)T + 1);
+    if (MULTI && (hdr >> 24 & kBulkFlag)) {  // a bulk: the warp publishes its roots
+      st_release(&P.seq[s], slot + P.cap);
+      state = 0;
+      events |= kBulkHeld;
+      splitk = hdr;
+      return 0;
+    }
     plen = (int)(hdr & 0xFFFFu);
     splitk = MULTI ? (hdr >> 24) & 0x3Fu : hdr >> 24;
     cur_inst = MULTI ? (hdr << 1) & 0x80000000u : 0u;  // the parity bit until start_task adds the instance
@@ -970,8 +1013,37 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     //    indices already reserved (below the cached tail) are polled
     if (state == 1 && slot < tl && ld_acquire(&P.seq[slot & (P.cap - 1u)]) == slot + 1u) {
       const uint32_t mask0 = take_task();
-      if (start_task(mask0)) state = 2;
-      else finish_task();
+      if (!MULTI || !(events & kBulkHeld)) {
+        if (start_task(mask0)) state = 2;
+        else finish_task();
+      }
+    }
+    if (MULTI) {
+      unsigned held = __ballot_sync(FULL, events & kBulkHeld);
+      const bool any = held != 0;
+      __syncwarp();  // the holders' words are read by all lanes
+      while (held) {
+        const int src = (tid & ~31) + __ffs(held) - 1;
+        held &= held - 1u;
+        const uint32_t first = s_lane[R::kCold + 3][src], hdr = s_lane[R::kCold + 5][src];
+        const uint32_t n = hdr & 0xFFFFu;
+        uint32_t t0 = 0;
+        if (lane == 0) t0 = atomicAdd(&ctl->tail, n);
+        t0 = __shfl_sync(FULL, t0, 0);
+        if ((uint32_t)lane < n) {
+          uint32_t root = first + (uint32_t)lane, kk = 0;
+          if (hdr >> 16 & 0xFFu) {
+            // the order is relative to the instance's first root
+            const uint32_t e = __ldcg(&P.order[root]);
+            root = P.inst_sub_base[P.subs[root].inst] + (e & 0x3FFFFFFu);
+            kk = e >> 26;
+          }
+          publish_root(P, t0 + (uint32_t)lane, root, 0, 0xF, kk | (hdr >> 24 & 0x40u));
+        }
+        __syncwarp();
+      }
+      events &= ~kBulkHeld;
+      if (any) continue;  // the holders claim again
     }
     // 3. nobody in the warp is searching: finished, failed or waiting
     const unsigned act = __ballot_sync(FULL, state == 2);

@@ -174,14 +174,15 @@ struct MultiBufs {
   int32_t *iter = nullptr, *fin = nullptr, *status = nullptr, *goal = nullptr, *ifv = nullptr;
   uint32_t *out = nullptr, *base = nullptr, *nsub = nullptr, *ioff = nullptr, *ilen = nullptr, *pair = nullptr;
   unsigned long long *icum = nullptr, *iter_nodes = nullptr, *loads = nullptr, *fin_ns = nullptr, *t0_ns = nullptr;
+  uint32_t *order = nullptr;  // [n_subs]: written and read by the kernel
   uint8_t *growth = nullptr;  // learned balancer: [n_subs][kGrowthSlacks] growth codes
   size_t cap_iter = 0, cap_fin = 0, cap_status = 0, cap_goal = 0, cap_ifv = 0, cap_out = 0,
          cap_base = 0, cap_nsub = 0, cap_ioff = 0, cap_ilen = 0, cap_icum = 0, cap_iter_nodes = 0, cap_loads = 0, cap_pair = 0,
-         cap_fin_ns = 0, cap_t0_ns = 0, cap_growth = 0;
+         cap_fin_ns = 0, cap_t0_ns = 0, cap_growth = 0, cap_order = 0;
   bool use_growth = false;  // the current launch has growth codes
   void release() {
     void *ptrs[] = {iter, fin,  status, goal, ifv,        out,   base,   nsub, pair,
-                    ioff, ilen, icum,   iter_nodes, loads, fin_ns, t0_ns, growth};
+                    ioff, ilen, icum,   iter_nodes, loads, fin_ns, t0_ns, growth, order};
     for (void *p : ptrs) cudaFree(p);
   }
 };
@@ -820,6 +821,7 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
     P.pair_nodes = (s->cfg.handback_nodes > 0 && n_inst * SP_PAIR_LANES <= (size_t)lanes) ? SP_PAIR_NODES : 0;
     P.iter_nodes = m.iter_nodes;
     P.sub_loads = m.loads;
+    P.order = m.order;
     P.inst_fin_ns = m.fin_ns;
     P.t_begin_ns = m.t0_ns;
     P.n_subs = (uint32_t)n_subs;
@@ -1178,7 +1180,8 @@ int solve_multi(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &inst,
       (rc = ensure(s, &m.iter_nodes, &m.cap_iter_nodes, ni * kMaxIters)) ||
       (rc = ensure(s, &m.loads, &m.cap_loads, 2 * std::max<size_t>(n_subs, 1))) ||
       (rc = ensure(s, &m.fin_ns, &m.cap_fin_ns, ni)) || (rc = ensure(s, &m.t0_ns, &m.cap_t0_ns, 1)) ||
-      (rc = ensure(s, &m.pair, &m.cap_pair, ni)))
+      (rc = ensure(s, &m.pair, &m.cap_pair, ni)) ||
+      (rc = ensure(s, &m.order, &m.cap_order, std::max<size_t>(n_subs, 1))))
     return rc;
   // uploads through one pinned staging buffer (asynchronous copies)
   auto bytes16 = [](const auto &v) { return (v.size() * sizeof(v[0]) + 15) & ~(size_t)15; };

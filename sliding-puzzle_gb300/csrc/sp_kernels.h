@@ -50,6 +50,7 @@ struct RoundParams {
                                       //   predicted below this many nodes (0: one at a time)
   unsigned long long *iter_nodes;     // [instance][kMaxIters] generated nodes
   unsigned long long *sub_loads;      // [2][n_subs] per-root loads of the last two iterations
+  uint32_t *order;                    // [n_subs] an instance's roots in publication order (search.cu)
   unsigned long long *inst_fin_ns;    // %globaltimer when the instance's answer became final
   unsigned long long *t_begin_ns;     // %globaltimer at the launch's first block start (atomicMin)
   uint32_t n_subs;
