@@ -682,6 +682,22 @@ int ensure_pool(sp_solver *s, size_t n_init) {
   return SP_OK;
 }
 
+// Limits and solution records for n instances, two of each per instance: the
+// device loop keeps one per iteration parity.
+int ensure_instances(sp_solver *s, size_t n) {
+  if (n <= s->inst_cap && s->d_limit && s->d_sol) return SP_OK;
+  if (s->d_limit) cudaFree(s->d_limit);
+  if (s->d_sol) cudaFree(s->d_sol);
+  s->d_limit = nullptr;
+  s->d_sol = nullptr;
+  s->inst_cap = 0;
+  const size_t c = std::max<size_t>(n, 64);
+  SP_CUDA(s, cudaMalloc(&s->d_limit, 2 * c * sizeof(int32_t)));
+  SP_CUDA(s, cudaMalloc(&s->d_sol, 2 * c * sizeof(Solution)));
+  s->inst_cap = c;
+  return SP_OK;
+}
+
 // The round's work: whole roots started as they are (direct, SubRoot ids in
 // publication order) and roots first expanded `flags` levels by the split
 // pre-pass.
@@ -1401,17 +1417,7 @@ int solve_impl(sp_solver *s, const uint8_t *tiles, int nin, sp_result *res) {
   size_t n_subs = 0;
   int rc = build_root_sets(s, tiles, inst, target, &n_subs);
   if (rc) return rc;
-  if (inst.size() > s->inst_cap || !s->d_limit) {
-    if (s->d_limit) cudaFree(s->d_limit);
-    if (s->d_sol) cudaFree(s->d_sol);
-    s->d_limit = nullptr;
-    s->d_sol = nullptr;
-    const size_t c = std::max<size_t>(inst.size(), 64);
-    // two entries per instance: the device loop keeps one per iteration parity
-    SP_CUDA(s, cudaMalloc(&s->d_limit, 2 * c * sizeof(int32_t)));
-    SP_CUDA(s, cudaMalloc(&s->d_sol, 2 * c * sizeof(Solution)));
-    s->inst_cap = c;
-  }
+  if ((rc = ensure_instances(s, inst.size()))) return rc;
   SP_CUDA(s, s->h_limits.reserve(inst.size()));
   s->stats.frontier_ms += ms_since(t_front);
   // persistent mode: the device loop; instances it hands back (large
@@ -1770,11 +1776,7 @@ int sp_dfs_round(sp_solver *s, const uint8_t *roots, const int32_t *depth, const
   if (rc) return rc;
   rc = ensure(s, &s->d_sub_nodes, &s->sub_nodes_cap, (size_t)n);
   if (rc) return rc;
-  if (!s->d_limit || s->inst_cap < 1) {
-    SP_CUDA(s, cudaMalloc(&s->d_limit, 64 * sizeof(int32_t)));
-    SP_CUDA(s, cudaMalloc(&s->d_sol, 64 * sizeof(Solution)));
-    s->inst_cap = 64;
-  }
+  if ((rc = ensure_instances(s, 1))) return rc;
   SP_CUDA(s, cudaMemcpyAsync(s->d_subs, subs.data(), subs.size() * sizeof(SubRoot), cudaMemcpyHostToDevice, s->st));
   SP_CUDA(s, cudaMemcpyAsync(s->d_limit, &limit, sizeof(int32_t), cudaMemcpyHostToDevice, s->st));
   SP_CUDA(s, cudaMemsetAsync(s->d_sol, 0, sizeof(Solution), s->st));
@@ -1815,11 +1817,7 @@ int sp_selftest_stall(sp_solver *s, int timeout_ms, int32_t *device_status) {
   if (rc) return rc;
   if ((rc = ensure(s, &s->d_subs, &s->subs_cap, 1)) || (rc = ensure(s, &s->d_sub_nodes, &s->sub_nodes_cap, 1)))
     return rc;
-  if (!s->d_limit || s->inst_cap < 1) {
-    SP_CUDA(s, cudaMalloc(&s->d_limit, 64 * sizeof(int32_t)));
-    SP_CUDA(s, cudaMalloc(&s->d_sol, 64 * sizeof(Solution)));
-    s->inst_cap = 64;
-  }
+  if ((rc = ensure_instances(s, 1))) return rc;
   // an empty pool, then one task counted as queued at index 0 that no
   // producer ever publishes: every lane that claims it waits for it
   SP_CUDA(s, launch_pool_init(s->d_tasks, nullptr, nullptr, nullptr, 0, s->d_seq, s->cap, s->d_ctl, nullptr, nullptr,
