@@ -23,7 +23,7 @@
 //    undoing a move restores the two overwritten values from the level's
 //    bytes instead of looking them up again;
 //  * generating a child and undoing a move share one code path (both slide
-//    one tile into the blank), and the warp's lanes are held together on it.
+//    one tile into the blank), without a branch between the two.
 //    Bound by issue and by table reads in flight.  Against the version with
 //    register boards and indices, whose lanes drifted apart (9-15 of 32
 //    active per instruction, 18-21 warp instructions per node; now 18 and
@@ -563,8 +563,9 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
   uint32_t rem = 0;              // moves still untried at the current node
   int hr = 0, hf = 0;            // h of the two partitions (Manhattan: hr alone)
   int budget = 0;                // a child of level k is entered when its h <= budget - k
-  int kstop = 0;                 // entering a child of this level is special: the first of a split
-                                 // task, else the last that the lane's stack and path can hold
+  int krare = 0;                 // entering a child of a level from here on needs a second look: the
+                                 // first level of a split task, levels beyond the shared ones or the
+                                 // last that the lane's stack and path can hold
   int groot = 0, plen = 0;
   int lo = 0;                    // donation: no level below lo has untried moves
   uint32_t cnt = 0;              // generated nodes not yet added to the task's counters
@@ -786,7 +787,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     rem = step_legal<W>(blank) & mask0;
     if (pre >= 0) rem &= ~(1u << (3 - pre));
     budget = limit - groot - 1;
-    kstop = splitk ? 0 : min(R::kMaxLev - 1, kMaxPath - plen);
+    krare = splitk ? 0 : min(min(R::kShared, R::kMaxLev - 1), kMaxPath - plen);
     k = 0;
     lo = 0;
     cnt = 0;
@@ -811,33 +812,31 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
   // they share one code path (lanes of a warp at different points of their
   // walks stay converged); only the child's table lookups, the f-test and
   // the level's word differ.
-  // `mates`: the lanes of the warp that take this step.  The warp syncs keep
-  // them on one path: without them the compiler gives generating and undoing
-  // lanes a copy each of the shared code.
+  // It is written with selects and reads that both kinds of lane make, one
+  // branch for what is entered and one for the rare cases: branches on the kind
+  // made the compiler give each kind a copy of the shared code (9 lanes per
+  // instruction; 18 with warp syncs in between, 19 and a tenth fewer
+  // instructions this way).
   // go on; task exhausted; child to hand to the pool; not searching
   enum { kStepOn, kStepDone, kStepEmit, kStepIdle };
-  auto step = [&](unsigned mates) -> int {
+  auto step = [&]() -> int {
     const bool gen = rem != 0;
-    // an undo: the level's moves, and the table values it had before the descent
-    uint32_t e = 0, vr = 0, vf = 0;
-    const int lev = gen ? k : k - 1;  // the level whose byte this step writes or reads
-    const uint32_t at = level_off(lev);
-    if (!gen) {
-      if (R::kDeep > 0 && lev >= R::kShared) {
-        const uint32_t w = deep[lev - R::kShared];
-        e = w & 0xFFu;
-        vr = (w >> 8) & 0xFFu;
-        vf = w >> 16;
-      } else {
-        e = mb[at];
-        if (PDB) {
-          vr = mb[at + 4u * BLOCK * R::kPlane];
-          vf = mb[at + 8u * BLOCK * R::kPlane];
-        }
-      }
+    const int lev = gen ? k : k - 1;  // the level whose bytes this step writes or reads
+    const uint32_t at = level_off(R::kDeep > 0 ? min(lev, R::kShared - 1) : lev);
+    // an undo: the level's moves, and the table values it had before the
+    // descent (a generating lane reads too, and drops it)
+    uint32_t e = mb[at], vr = 0, vf = 0;
+    if (PDB) {
+      vr = mb[at + 4u * BLOCK * R::kPlane];
+      vf = mb[at + 8u * BLOCK * R::kPlane];
     }
-    __syncwarp(mates);
-    const uint32_t dm = gen ? first_move(rem) : e >> 4;  // the blank's move this step
+    if (R::kDeep > 0 && lev >= R::kShared) {
+      const uint32_t w = deep[lev - R::kShared];
+      e = w & 0xFFu;
+      vr = (w >> 8) & 0xFFu;
+      vf = w >> 16 & 0xFFu;
+    }
+    const uint32_t dm = gen ? first_move(rem) : e >> 4 & 3u;  // the blank's move this step
     rem &= rem - 1u;
     cnt += gen;
     const int from = blank + step_delta<W>(dm);
@@ -866,11 +865,12 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
         oldf = mb[(R::kVal + 1) * 4 * BLOCK + qf];
         child = s_rem[(uint32_t)from * 4u + dm];
       }
-      if (gen) {
-        vr = lookup(W == 4 ? nr & 0x3FFFFFu : nr);
-        vf = lookup(W == 4 ? nf & 0x3FFFFFu : nf);
-      }
-      __syncwarp(mates);
+      // undoing lanes read entry 0 of the first table: one sector for all of
+      // them, and the warp stays on one path
+      const uint32_t tr = lookup(!gen ? 0u : W == 4 ? nr & 0x3FFFFFu : nr);
+      const uint32_t tf = lookup(!gen ? 0u : W == 4 ? nf & 0x3FFFFFu : nf);
+      vr = gen ? tr : vr;
+      vf = gen ? tf : vf;
       nhr = hr + (int)(vr - oldr);
       nhf = hf + (int)(vf - oldf);
     } else {
@@ -894,31 +894,28 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
       mb[boff] = (uint8_t)t;
       boff = foff;
       blank = from;
-      if (gen) {
-        const uint32_t up = rem | (3u - dm) << 4;
-        if (R::kDeep > 0 && lev >= R::kShared) {
-          deep[lev - R::kShared] = up | oldr << 8 | oldf << 16;
-        } else {
-          mb[at] = (uint8_t)up;
-          if (PDB) {
-            mb[at + 4u * BLOCK * R::kPlane] = (uint8_t)oldr;
-            mb[at + 8u * BLOCK * R::kPlane] = (uint8_t)oldf;
-          }
+      const uint32_t up = rem | (3u - dm) << 4;
+      if (gen && (R::kDeep == 0 || lev < R::kShared)) {
+        mb[at] = (uint8_t)up;
+        if (PDB) {
+          mb[at + 4u * BLOCK * R::kPlane] = (uint8_t)oldr;
+          mb[at + 8u * BLOCK * R::kPlane] = (uint8_t)oldf;
         }
-        ++k;
-        rem = child;
+      }
+      rem = gen ? child : e & 15u;
+      k = gen ? lev + 1 : lev;
+      if (gen && (nh == 0 || lev >= krare)) {
+        if (R::kDeep > 0 && lev >= R::kShared) deep[lev - R::kShared] = up | oldr << 8 | oldf << 16;
         if (nh == 0) record_goal();
-        if (lev == kstop) {
-          // split task with `splitk` levels left: this child (already counted
-          // as generated) becomes a task of its own with one level fewer
-          // (published outside the step loop), so a heavy root is split
-          // breadth-first by many lanes; the lane then steps back
-          ev = splitk ? kStepEmit : kStepDone;
-          if (!splitk) set_error(SP_ERR_STACK_OVERFLOW, (uint32_t)(plen + lev));
+        // split task with `splitk` levels left: this child (already counted
+        // as generated) becomes a task of its own with one level fewer
+        // (published outside the step loop), so a heavy root is split
+        // breadth-first by many lanes; the lane then steps back
+        if (splitk && lev == 0) ev = kStepEmit;
+        if (lev >= min(R::kMaxLev - 1, kMaxPath - plen)) {
+          set_error(SP_ERR_STACK_OVERFLOW, (uint32_t)(plen + lev));
+          ev = kStepDone;
         }
-      } else {
-        --k;
-        rem = e & 15u;
       }
     }
     return ev;
@@ -1082,11 +1079,10 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     uint32_t taken = 0;
     for (int s = 0; s < P.steps; ++s) {
       const bool go = ev == kStepOn && (rem | (uint32_t)k) != 0u;  // else: nothing left of the task
-      const unsigned mates = __ballot_sync(FULL, go);
-      if (!mates) break;
+      if (!__any_sync(FULL, go)) break;
       if (go) {
         ++taken;
-        ev = step(mates);
+        ev = step();
       }
     }
     if (ev == kStepOn && (rem | (uint32_t)k) == 0u) ev = kStepDone;
