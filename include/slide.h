@@ -209,7 +209,7 @@ int sp_dfs_round(sp_solver *s, const uint8_t *roots, const int32_t *depth,
  * sp_dfs_round, d_nodes[n] and d_found[1] receive its outputs; stream is a
  * cudaStream_t (NULL = default stream).  The call is synchronous: it copies
  * the device status back and returns after the stream has drained.  Scratch
- * lives in a fixed device array of about 7 MB that every GPU loading the
+ * lives in a fixed device array of about 12 MB that every GPU loading the
  * library keeps until exit; n above 16384 roots returns SP_ERR_CAPACITY
  * before anything is launched.  Calls share that array and each re-writes
  * what must start clean: calls overlapping on the GPU race, so serialise

@@ -8,7 +8,7 @@
 // unbounded.  They pass device buffers for the inputs and outputs;
 // everything else the round needs lives in one file-scope device array of
 // fixed size, g_noalloc_scratch below.  Every GPU that loads the library
-// holds that array (kNoAllocScratchBytes, about 7 MB) until the process
+// holds that array (kNoAllocScratchBytes, about 12 MB) until the process
 // exits.
 //
 // Limits and sharing: at most kNoAllocMaxRoots roots per call and a task

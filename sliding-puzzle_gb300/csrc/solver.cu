@@ -237,8 +237,9 @@ struct sp_solver {
   uint32_t last_emitted = 0;
   // split pre-pass buffers
   uint32_t *d_cnt = nullptr;  // [level a, level b, emitted, error]
-  Task *d_split_a = nullptr, *d_split_b = nullptr, *d_emit = nullptr;
-  size_t split_cap_a = 0, split_cap_b = 0, emit_cap = 0;
+  uint2 *d_split_roots = nullptr;
+  Task *d_split_a = nullptr, *d_split_b = nullptr;
+  size_t split_cap_roots = 0, split_cap_a = 0, split_cap_b = 0;
   // device task pool
   Task *d_tasks = nullptr;
   uint32_t *d_seq = nullptr;
@@ -259,7 +260,7 @@ struct sp_solver {
   size_t boards_cap = 0, h_cap = 0;
   // pinned staging
   Pinned<uint32_t> h_direct;
-  Pinned<Task> h_split;
+  Pinned<uint2> h_split;  // (SubRoot, levels)
   Pinned<unsigned long long> h_sub_nodes;
   Pinned<Solution> h_sols;
   Pinned<PoolCtl> h_ctl;
@@ -699,17 +700,16 @@ int ensure_instances(sp_solver *s, size_t n) {
 }
 
 // The round's work: whole roots started as they are (direct, SubRoot ids in
-// publication order) and roots first expanded `flags` levels by the split
-// pre-pass.
+// publication order) and roots first expanded some levels by the split
+// pre-pass (written by the static planner straight into h_split).
 struct RoundPlan {
   std::vector<uint32_t> direct;
-  std::vector<Task> split;
   // the static planner writes straight into the solver's pinned staging
-  // buffers (h_direct, h_split) instead; the vectors above stay empty
+  // buffers (h_direct, h_split) instead; the vector above stays empty
   bool staged = false;
   size_t staged_direct = 0, staged_split = 0;
   size_t n_direct() const { return staged ? staged_direct : direct.size(); }
-  size_t n_split() const { return staged ? staged_split : split.size(); }
+  size_t n_split() const { return staged ? staged_split : 0; }
   size_t level_bound = 0;  // nodes one split level can hold
   size_t emit_bound = 0;   // pieces the split pre-pass can emit
   int max_k = 0;
@@ -756,20 +756,12 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
   s->h_cnt.p[1] = s->h_cnt.p[2] = s->h_cnt.p[3] = 0;
   SP_CUDA(s, cudaMemcpyAsync(s->d_cnt, s->h_cnt.p, 4 * sizeof(uint32_t), cudaMemcpyHostToDevice, s->st));
   if (n_split) {
-    const size_t lb = std::max(plan.level_bound, n_split);
-    rc = ensure(s, &s->d_split_a, &s->split_cap_a, lb);
-    if (rc) return rc;
-    rc = ensure(s, &s->d_split_b, &s->split_cap_b, lb);
-    if (rc) return rc;
-    rc = ensure(s, &s->d_emit, &s->emit_cap, std::max<size_t>(plan.emit_bound, 1));
-    if (rc) return rc;
-    if (!plan.staged) {
-      SP_CUDA(s, s->h_split.reserve(n_split));
-      memcpy(s->h_split.p, plan.split.data(), n_split * sizeof(Task));
-    }
-    SP_CUDA(s, cudaMemcpyAsync(s->d_split_a, s->h_split.p, n_split * sizeof(Task),
-                               cudaMemcpyHostToDevice, s->st));
-    s->stats.h2d_bytes += n_split * sizeof(Task);
+    const size_t lb = std::max<size_t>(plan.level_bound, 1);
+    if ((rc = ensure(s, &s->d_split_roots, &s->split_cap_roots, n_split)) ||
+        (rc = ensure(s, &s->d_split_a, &s->split_cap_a, lb)) || (rc = ensure(s, &s->d_split_b, &s->split_cap_b, lb)))
+      return rc;
+    SP_CUDA(s, cudaMemcpyAsync(s->d_split_roots, s->h_split.p, n_split * sizeof(uint2), cudaMemcpyHostToDevice, s->st));
+    s->stats.h2d_bytes += n_split * sizeof(uint2);
   }
   SP_CUDA(s, cudaEventRecord(s->ev0, s->st));
   for (int l = 0; l < plan.max_k; ++l) {
@@ -782,20 +774,21 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
     A.pdb = s->d_pdb;
     A.sub_nodes = s->d_sub_nodes;
     A.sol = s->d_sol;
+    A.roots = l == 0 ? s->d_split_roots : nullptr;
     A.in = cur ? s->d_split_b : s->d_split_a;
     A.n_in = s->d_cnt + cur;
     A.next = nxt ? s->d_split_b : s->d_split_a;
     A.n_next = s->d_cnt + nxt;
     A.cap_next = (uint32_t)(nxt ? s->split_cap_b : s->split_cap_a);
-    A.out = s->d_emit;
+    A.out = s->d_tasks;
     A.n_out = s->d_cnt + 2;
-    A.cap_out = (uint32_t)s->emit_cap;
+    A.cap_out = s->cap;
     A.error = (int32_t *)(s->d_cnt + 3);
     SP_CUDA(s, launch_split_level(s->w, s->heur == SP_HEUR_PDB, s->num_sms, A, s->st));
     s->stats.kernel_launches += 1;
   }
-  SP_CUDA(s, launch_pool_init(s->d_tasks, s->d_emit, plan.max_k ? s->d_cnt + 2 : nullptr, s->d_direct, n_direct,
-                              s->d_seq, s->cap, s->d_ctl, multi ? s->d_subs : nullptr, multi ? s->mb.iter : nullptr,
+  SP_CUDA(s, launch_pool_init(s->d_tasks, plan.max_k ? s->d_cnt + 2 : nullptr, s->d_direct, n_direct, s->d_seq,
+                              s->cap, s->d_ctl, multi ? s->d_subs : nullptr, multi ? s->mb.iter : nullptr,
                               s->st));
   RoundParams P{};
   P.subs = s->d_subs;
@@ -1044,7 +1037,7 @@ int plan_round(sp_solver *s, std::vector<Instance> &inst, const std::vector<int3
   SP_CUDA(s, s->h_direct.reserve(std::max<size_t>(nd, 1)));
   SP_CUDA(s, s->h_split.reserve(std::max<size_t>(nsp, 1)));
   uint32_t *out_direct = s->h_direct.p;
-  Task *out_split = s->h_split.p;
+  uint2 *out_split = s->h_split.p;
   plan.staged = true;
   plan.staged_direct = nd;
   plan.staged_split = nsp;
@@ -1054,11 +1047,7 @@ int plan_round(sp_solver *s, std::vector<Instance> &inst, const std::vector<int3
       const int kk = std::min((int)k[j], kmax);
       const uint32_t sub = inst[i].sub_base + (uint32_t)q;
       if (kk > 0) {
-        Task t{};
-        t.sub = sub;
-        t.mask = 0xF;
-        t.flags = (uint8_t)kk;
-        out_split[cs[bucket[j]]++] = t;
+        out_split[cs[bucket[j]]++] = make_uint2(sub, (uint32_t)kk);
       } else {
         out_direct[cd[bucket[j]]++] = sub;
       }
@@ -1622,7 +1611,7 @@ void sp_destroy(sp_solver *s) {
   cudaFree(s->d_cnt);
   cudaFree(s->d_split_a);
   cudaFree(s->d_split_b);
-  cudaFree(s->d_emit);
+  cudaFree(s->d_split_roots);
   s->mb.release();
   s->fb.release();
   if (s->ev0) cudaEventDestroy(s->ev0);
@@ -1820,7 +1809,7 @@ int sp_selftest_stall(sp_solver *s, int timeout_ms, int32_t *device_status) {
   if ((rc = ensure_instances(s, 1))) return rc;
   // an empty pool, then one task counted as queued at index 0 that no
   // producer ever publishes: every lane that claims it waits for it
-  SP_CUDA(s, launch_pool_init(s->d_tasks, nullptr, nullptr, nullptr, 0, s->d_seq, s->cap, s->d_ctl, nullptr, nullptr,
+  SP_CUDA(s, launch_pool_init(s->d_tasks, nullptr, nullptr, 0, s->d_seq, s->cap, s->d_ctl, nullptr, nullptr,
                               s->st));
   SP_CUDA(s, s->h_cnt.reserve(4));
   s->h_cnt.p[0] = 1;

@@ -96,15 +96,22 @@ struct SubRoot {
 static_assert(sizeof(SubRoot) == 32, "SubRoot layout");
 
 // Unit of work in the device task pool: the node reached from SubRoot `sub`
-// by `plen` moves, restricted to the first-level moves in `mask`.
-struct Task {
+// by `plen` moves, restricted to the first-level moves in `mask`.  A task
+// below its root (plen > 0) carries its board, so that its claimant need not
+// replay the path; of a root itself only mask, sub, plen and flags count.
+struct alignas(16) Task {
+  uint8_t board[kMaxN];
+  uint8_t blank, g;
+  uint8_t mask;     // plen > 0: legal moves only, none of them the reverse
   uint32_t sub;
-  uint16_t plen;
-  uint8_t mask;
+  uint8_t plen;
   uint8_t flags;
+  int16_t budget;   // plen > 0: a child is entered when its h <= budget
   uint32_t path[kPathWords];
+  uint32_t pad;
 };
-static_assert(sizeof(Task) == 48, "Task layout");
+static_assert(sizeof(Task) == 80, "Task layout");
+constexpr int kMaxBudget = 30000;  // no sum of table bytes and moves comes near
 
 // One goal per instance: moves below its SubRoot.  `best` is
 // 0xFFFFFFFF - (shortest absolute goal depth seen), 0 when none, so that a

@@ -69,15 +69,17 @@ cudaError_t launch_search_round(int w, bool pdb, int block, int blocks_per_sm, i
 // The whole threshold loop of a batch in one launch (multi-iteration mode).
 cudaError_t launch_search_multi(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
                                 const RoundParams &P, cudaStream_t st, int *grid_out);
-// Publish the round's tasks (split pieces first, then the direct tasks) and
-// reset the pool control block.
+// Publish the round's tasks and reset the pool control block: the split
+// pieces (*n_emit of them, 0 when null), which the pre-pass has written to the
+// ring's first slots, then the direct tasks.
 // Multi-iteration mode passes subs and inst_iter: each direct task then
 // carries its instance's iteration parity.
-cudaError_t launch_pool_init(Task *tasks, const Task *emit, const uint32_t *n_emit, const uint32_t *direct,
-                             uint32_t n_direct, uint32_t *seq, uint32_t cap, PoolCtl *ctl, const SubRoot *subs,
-                             const int32_t *inst_iter, cudaStream_t st);
+cudaError_t launch_pool_init(Task *tasks, const uint32_t *n_emit, const uint32_t *direct, uint32_t n_direct,
+                             uint32_t *seq, uint32_t cap, PoolCtl *ctl, const SubRoot *subs, const int32_t *inst_iter,
+                             cudaStream_t st);
 
-// Split pre-pass: one breadth-first level over `in` (count *n_in).
+// Split pre-pass: one breadth-first level over `in`, or over `roots` (SubRoot,
+// levels) at the first one (count *n_in).
 struct SplitArgs {
   const SubRoot *subs;
   const int32_t *inst_limit;
@@ -85,6 +87,7 @@ struct SplitArgs {
   const uint8_t *pdb;
   unsigned long long *sub_nodes;
   Solution *sol;
+  const uint2 *roots;
   const Task *in;
   const uint32_t *n_in;
   Task *next;
