@@ -437,12 +437,14 @@ constexpr int threads_per_sm(int w, bool pdb) { return pdb && w == 4 ? 1024 : 76
 //           width 5: base in bit 28, the values as bytes of two more words)
 //   cold    data of rare events
 //   level   per level of the walk a byte with the moves still untried there
-//           (bits 0-3) and the reverse of the move taken (bits 4-5) and, for
+//           (bits 0-3), the reverse of the move taken (bits 4-5) and whether
+//           it made h larger (bit 6, rounds alone) and, for
 //           the PDB, a byte in each of two more planes: the regular and the
 //           reflected table value that move overwrote; PDB levels beyond the
 //           shared ones are in local memory
 // The level bytes hold what an undo needs, so it neither recomputes the
 // move mask nor reads a table, and donating a level is clearing its mask.
+constexpr uint32_t kHarder = 64u;
 template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
 struct LaneRows {
   static constexpr int N = W * W;
@@ -569,6 +571,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
                                  // last that the lane's stack and path can hold
   int groot = 0, plen = 0;
   int lo = 0;                    // donation: no level below lo has untried moves
+  int lo_slack = 0;              // the limit less f at level lo (kHarder)
   uint32_t cnt = 0;              // generated nodes not yet added to the task's counters
   // Rare per-lane events, flags in a register and their data in shared memory:
   //  * kAdvance: the lane finished an instance's iteration; the warp advances
@@ -821,6 +824,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     rem = step_legal<W>(blank) & mask;
     if (pre >= 0) rem &= ~(1u << (3 - pre));
     krare = splitk ? 0 : min(min(R::kShared, R::kMaxLev - 1), kMaxPath - plen);
+    lo_slack = budget + 1 - h;
     return h <= budget + 1;
   };
   auto record_goal = [&]() {
@@ -908,7 +912,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
       child = m & 15u;
       nhr = hr + (int)((m >> 3) & 2u) - 1;
     }
-    const int nh = PDB ? max(nhr, nhf) : nhr;
+    const int nh = PDB ? max(nhr, nhf) : nhr, h0 = PDB ? max(hr, hf) : hr;
     int ev = kStepOn;
     if (!gen || nh <= budget - k) {  // else: generated, not entered
       if (PDB) {
@@ -924,7 +928,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
       mb[boff] = (uint8_t)t;
       boff = foff;
       blank = from;
-      const uint32_t up = rem | (3u - dm) << 4;
+      const uint32_t up = rem | (3u - dm) << 4 | (!MULTI && nh > h0 ? kHarder : 0u);
       if (gen && (R::kDeep == 0 || lev < R::kShared)) {
         mb[at] = (uint8_t)up;
         if (PDB) {
@@ -956,16 +960,18 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
   auto find_donation = [&](uint32_t &mask_out) -> int {
     // resume at the first level not yet seen exhausted (`lo`): a level only
     // loses untried moves during a task, so the walk never needs to look
-    // below it again; above the current depth it restarts at k
-    int j = min(lo, k), found = -1;
+    // below it again, and has nothing left when it has stepped back past it
+    if (k < lo) return -1;
+    int j = lo, found = -1;
     const int last = min(k, budget + 1 - P.min_slack);
     for (; j <= last; ++j) {
-      const uint32_t un = j == k ? rem : level_get(j) & 15u;
-      if (un) {
-        mask_out = un;
+      const uint32_t e = j == k ? rem : level_get(j);
+      if (e & 15u) {
+        mask_out = e & 15u;
         found = j;
         break;
       }
+      if (e & kHarder) lo_slack -= 2;
     }
     lo = min(j, k);
     return found;
@@ -1104,7 +1110,12 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     // searches, and the vote brings them back together
     int ev = state == 2 ? kStepOn : kStepIdle;
     uint32_t taken = 0;
-    for (int s = 0; s < P.steps; ++s) {
+    // A round's passes are a quarter longer than the device loop's, where the
+    // next iteration waits for the last one's tasks (32 / 40 / 48 steps: 100
+    // random 15-puzzles 17.4 / 16.9 / 16.9 ms, 2048 24-puzzle roots 11.8 / 11.3
+    // / 11.2, 50 24-puzzles 12.7 / 12.9 / 12.9).
+    const int steps = MULTI ? P.steps : P.steps + P.steps / 4;
+    for (int s = 0; s < steps; ++s) {
       const bool go = ev == kStepOn && (rem | (uint32_t)k) != 0u;  // else: nothing left of the task
       if (!__any_sync(FULL, go)) break;
       if (go) {
@@ -1115,7 +1126,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
     if (ev == kStepOn && (rem | (uint32_t)k) == 0u) ev = kStepDone;
     taken = __reduce_add_sync(FULL, taken);
     if (lane == 0) {
-      ws.slots += 32ull * (unsigned long long)P.steps;
+      ws.slots += 32ull * (unsigned long long)steps;
       ws.steps += taken;
     }
     if (state == 2) {
@@ -1147,13 +1158,27 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_
       uint32_t dmask = 0;
       int lev = (state == 2) ? find_donation(dmask) : -1;
       if (lev >= 0 && plen + lev > kMaxPath) lev = -1;  // prefix would not fit a record
-      // donors: lanes whose open level is within one of the warp's shallowest,
-      // at most `allowed` of them (more when the shortfall is large)
-      const unsigned key = lev >= 0 ? (unsigned)lev : 0xFFFFFFFFu;
+      // donors: the lanes with about the largest parts, at most `allowed` of
+      // them (more when the shortfall is large).  A part's size goes by its
+      // node's slack and the moves left at it: two of slack are worth six moves.
+      // In the device loop, where iterations are small and the next one waits
+      // for their last task, it goes by the level in the task alone, which
+      // spreads the newest tasks first.
+      // Rounds, by level / moves left / 1, 2, 3 or 8 slack + moves left: 16384
+      // 24-puzzle roots 84.5 / 71.1 / 71.3 / 70.1 / 69.9 / - ms, 2048 of them
+      // by Manhattan 22.0 / 12.9 / 12.1 / 11.8 / 11.7 / 12.1, 100 random
+      // 15-puzzles 19.1 / 18.3 / 17.5 / 17.4 / 17.3 / 18.8 (a task then holds
+      // 40 % more nodes).  The device loop on 50 24-puzzles by level 2.3, by
+      // moves left 2.9, by both 2.6.
+      constexpr int kScoreSlack = 3;
+      constexpr unsigned kNear = MULTI ? 1u : 4u;
+      const unsigned key = lev < 0 ? 0xFFFFFFFFu
+                           : MULTI ? (unsigned)lev
+                                   : (1u << 24) - (unsigned)(kScoreSlack * min(lo_slack, 1 << 16) + min(budget, 1 << 16) - lev);
       const unsigned best = __reduce_min_sync(FULL, key);
       const uint32_t shortfall = hd + P.reserve - tl;
       const unsigned allowed = min((unsigned)SP_MAX_DONORS, 1u + shortfall / P.spread);
-      const unsigned cand = __ballot_sync(FULL, lev >= 0 && (unsigned)lev <= best + 1u);
+      const unsigned cand = __ballot_sync(FULL, lev >= 0 && key <= best + kNear);
       const unsigned rank = __popc(cand & ((1u << lane) - 1u));
       const bool donor = ((cand >> lane) & 1u) && rank < allowed && !(events & kDebt);
       const unsigned donors = __ballot_sync(FULL, donor);
