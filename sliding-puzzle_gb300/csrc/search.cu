@@ -426,7 +426,10 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
 // ms, but a batch of 50 12.1 against 11.5 ms).  Manhattan reads no tables:
 // 768 or 1024 threads measure alike.
 constexpr int kSharedPerSm = 192 * 1024;
-constexpr int threads_per_sm(int w, bool pdb) { return pdb && w == 4 ? 1024 : 768; }
+// The device loop is bound by its chains of small iterations, not by reads in
+// flight, and would spill 188 bytes at 64 registers: 768 threads (100 random
+// 15-puzzles 17.2 -> 17.0 ms).
+constexpr int threads_per_sm(int w, bool pdb, bool multi) { return pdb && w == 4 && !multi ? 1024 : 768; }
 
 // What a lane keeps in shared memory: 32-bit words, one column per lane
 // ([row][thread]), so that a lane only ever touches its own bank whatever
@@ -459,7 +462,7 @@ struct LaneRows {
   static constexpr int kMoveTable = PDB ? (W == 4 ? 8 * 4 * N * N : 8 * N * N + 4 * N) : 4 * N * N;
   static constexpr int kFixed = kMoveTable + 64 + (MULTI ? BLOCK * 4 : 4) + BLOCK / 32 * 64;
   // shared levels: what fits beside the rest (1 KB is reserved per block)
-  static constexpr int kBudget = kSharedPerSm / (threads_per_sm(W, PDB) / BLOCK) - 1024;
+  static constexpr int kBudget = kSharedPerSm / (threads_per_sm(W, PDB, MULTI) / BLOCK) - 1024;
   static constexpr int kFit = (kBudget - kFixed) / (4 * BLOCK) - kLevel;
   static constexpr int kShared = PDB && kFit / 3 * 4 < kMaxLev ? kFit / 3 * 4 : kMaxLev;
   static constexpr int kDeep = kMaxLev - kShared;
@@ -476,7 +479,7 @@ struct WarpState {
 static_assert(sizeof(WarpState) == 64, "WarpState layout");
 
 template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
-__global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB) / BLOCK) search_round_kernel(RoundParams P) {
+__global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) search_round_kernel(RoundParams P) {
   using R = LaneRows<W, PDB, BLOCK, WORDS, MULTI>;
   constexpr int N = W * W;
   constexpr unsigned FULL = 0xffffffffu;
