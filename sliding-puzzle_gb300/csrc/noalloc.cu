@@ -245,7 +245,7 @@ extern "C" int sp_dfs_round_md_noalloc(int width, const uint8_t *d_roots, const 
     P.poll_ns = 2000;
     const uint32_t lanes = (uint32_t)num_sms * 1024u;
     P.reserve = lanes / 16u;
-    P.spread = lanes / 32u;
+    P.spread = lanes / 64u;
     int grid = 0;
     if (launch_search_round(width, false, 256, 0, num_sms, P, st, &grid) != cudaSuccess) return SP_ERR_CUDA;
   }

@@ -1117,7 +1117,13 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) 
     // next iteration waits for the last one's tasks (32 / 40 / 48 steps: 100
     // random 15-puzzles 17.4 / 16.9 / 16.9 ms, 2048 24-puzzle roots 11.8 / 11.3
     // / 11.2, 50 24-puzzles 12.7 / 12.9 / 12.9).
-    const int steps = MULTI ? P.steps : P.steps + P.steps / 4;
+    // While three lanes in four wait, they are half as long: issue slots are
+    // free and what counts is how fast work spreads (32 / 16 / 8 steps then: 50
+    // 24-puzzles 12.8 / 12.3 / 12.6, one random 15-puzzle 1.60 / 1.52 / 1.51,
+    // 100 Manhattan walks 9.41 / 9.42 / 9.58; from half of the lanes on, 12.2,
+    // 1.41 and 9.65 with 16 steps).
+    int steps = MULTI ? P.steps : P.steps + P.steps / 4;
+    if ((int32_t)(hd - tl) > (int32_t)(48u * P.spread)) steps = (P.steps + 1) / 2;
     for (int s = 0; s < steps; ++s) {
       const bool go = ev == kStepOn && (rem | (uint32_t)k) != 0u;  // else: nothing left of the task
       if (!__any_sync(FULL, go)) break;
