@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) 
     write_path(len, [&](int wi, uint32_t v) { D->path[wi] = v; });
     st_release(&P.seq[t & (P.cap - 1u)], t + 1u);
   };
-  auto lookup = [&](uint32_t off) -> uint32_t { return __ldcg(P.pdb + off); };
+  auto lookup = [&](uint32_t off) -> uint32_t { return __ldg(P.pdb + off); };
   // h of the lane's board (its blank byte 0) from nothing: pattern indices
   // and table values too
   auto full_h = [&]() -> int {
