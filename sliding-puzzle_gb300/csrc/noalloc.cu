@@ -246,8 +246,8 @@ extern "C" int sp_dfs_round_md_noalloc(int width, const uint8_t *d_roots, const 
     const uint32_t lanes = (uint32_t)num_sms * 1024u;
     P.reserve = lanes / 16u;
     P.spread = lanes / 64u;
-    int grid = 0;
-    if (launch_search_round(width, false, 256, 0, num_sms, P, st, &grid) != cudaSuccess) return SP_ERR_CUDA;
+    int lanes_run = 0;
+    if (launch_search_round(width, false, 256, 0, num_sms, P, st, &lanes_run) != cudaSuccess) return SP_ERR_CUDA;
   }
   noalloc_finish_kernel<<<1, 1, 0, st>>>(base, d_found);
   if (!launched(1)) return SP_ERR_CUDA;

@@ -417,19 +417,27 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
 // Resident threads per SM that the search kernels are compiled for, and the
 // shared memory that these may take together.  The PDB search is bound by its
 // table reads in flight: a read that misses L1 holds an L1 line until L2
-// answers, so the part of the SM's 256 KB that is left to L1 limits them.  At
-// 228 KB of shared memory (28 KB of L1) a batch of 4096 15-puzzles took 288
-// ms and a 16384-root round of the 24-puzzle 148 ms, at up to 196 KB 247 and
-// 102 ms, and only with the larger L1 do more warps pay: 1024 threads (64
-// registers, nothing spilled) 220 ms.  The 24-puzzle's rows are longer: at
-// 1024 threads its shared levels would shrink from 48 to 28 (100 against 102
-// ms, but a batch of 50 12.1 against 11.5 ms).  Manhattan reads no tables:
-// 768 or 1024 threads measure alike.
-constexpr int kSharedPerSm = 192 * 1024;
+// answers, so the part of the SM's 256 KB that is left to L1 limits them, and
+// more warps pay only with a larger L1.  A round's kernel therefore is one
+// block per SM: the move tables are there once instead of three or four times,
+// and 164 KB of shared memory, 92 KB of L1, hold as many threads and about as
+// many shared levels as 192 KB did in blocks of 256 (4096 15-puzzles: 100 /
+// 132 / 164 / 196 KB 207 / 183 / 156 / 161 ms, blocks of 256 166 ms and at 228
+// KB 260; 16384 24-puzzle roots 78.6 / 74.6 / 63.7 / 67.9, blocks of 256
+// 68.2).  Threads, 15-puzzle: 768 / 896 / 1024 166 / 157 / 156 ms;
+// 24-puzzle, whose rows are longer, so that more threads leave it fewer shared
+// levels: 640 / 768 / 896 / 1024 65.3 / 63.8 / 70.3 / 72.7.
+// Blocks of 128 and 256 threads stay for a caller that asks for them or for a
+// number of blocks per SM.  Manhattan reads no tables: 768 or 1024 threads
+// measure alike.
 // The device loop is bound by its chains of small iterations, not by reads in
 // flight, and would spill 188 bytes at 64 registers: 768 threads (100 random
 // 15-puzzles 17.2 -> 17.0 ms).
-constexpr int threads_per_sm(int w, bool pdb, bool multi) { return pdb && w == 4 && !multi ? 1024 : 768; }
+constexpr int big_block(int w) { return w == 4 ? 1024 : 768; }
+constexpr int shared_per_sm(int block) { return (block > 256 ? 164 : 192) * 1024; }
+constexpr int blocks_on_sm(int w, bool pdb, bool multi, int block) {
+  return block > 256 ? 1 : (pdb && w == 4 && !multi ? 1024 : 768) / block;
+}
 
 // What a lane keeps in shared memory: 32-bit words, one column per lane
 // ([row][thread]), so that a lane only ever touches its own bank whatever
@@ -457,12 +465,14 @@ struct LaneRows {
   static constexpr int kIdx = kBoard + (N + 3) / 4;
   static constexpr int kVal = kIdx + (PDB ? 2 * kPat : 0);
   static constexpr int kCold = kVal + (PDB && W == 5 ? 2 : 0);
-  static constexpr int kLevel = kCold + 6;
+  static constexpr int kSub = kCold, kSplit = kCold + 1, kDebtAt = kCold + 2, kDebtSub = kCold + 3;
+  static constexpr int kInst = MULTI ? kCold + 4 : kSub, kDone = MULTI ? kCold + 5 : kSub;  // device loop alone
+  static constexpr int kLevel = kCold + (MULTI ? 6 : 4);
   // move tables of the block (bytes), pool cache and publication buckets
   static constexpr int kMoveTable = PDB ? (W == 4 ? 8 * 4 * N * N : 8 * N * N + 4 * N) : 4 * N * N;
   static constexpr int kFixed = kMoveTable + 64 + (MULTI ? BLOCK * 4 : 4) + BLOCK / 32 * 64;
   // shared levels: what fits beside the rest (1 KB is reserved per block)
-  static constexpr int kBudget = kSharedPerSm / (threads_per_sm(W, PDB, MULTI) / BLOCK) - 1024;
+  static constexpr int kBudget = shared_per_sm(BLOCK) / blocks_on_sm(W, PDB, MULTI, BLOCK) - 1024;
   static constexpr int kFit = (kBudget - kFixed) / (4 * BLOCK) - kLevel;
   static constexpr int kShared = PDB && kFit / 3 * 4 < kMaxLev ? kFit / 3 * 4 : kMaxLev;
   static constexpr int kDeep = kMaxLev - kShared;
@@ -479,7 +489,7 @@ struct WarpState {
 static_assert(sizeof(WarpState) == 64, "WarpState layout");
 
 template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
-__global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) search_round_kernel(RoundParams P) {
+__global__ void __launch_bounds__(BLOCK, blocks_on_sm(W, PDB, MULTI, BLOCK)) search_round_kernel(RoundParams P) {
   using R = LaneRows<W, PDB, BLOCK, WORDS, MULTI>;
   constexpr int N = W * W;
   constexpr unsigned FULL = 0xffffffffu;
@@ -552,13 +562,12 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) 
   // levels beyond the shared ones, their three bytes in a word
   uint32_t prefix[kPathWords], start_board[7], deep[R::kDeep > 0 ? R::kDeep : 1] = {0};
   WarpState &ws = s_warp[tid >> 5];
-  uint32_t *const s_cold0 = s_lane[R::kCold], *const s_cold1 = s_lane[R::kCold + 1],
-           *const s_cold2 = s_lane[R::kCold + 2];
+  uint32_t *const s_cold0 = s_lane[R::kDone], *const s_cold1 = s_lane[R::kDebtAt],
+           *const s_cold2 = s_lane[R::kDebtSub];
   // the task's SubRoot; its instance (multi-iteration mode: bit 31 = the
   // parity of the task's iteration); its split levels (a split task hands
   // every node at relative depth 1 to the pool)
-  uint32_t &sub = s_lane[R::kCold + 3][tid], &cur_inst = s_lane[R::kCold + 4][tid],
-           &splitk = s_lane[R::kCold + 5][tid];
+  uint32_t &sub = s_lane[R::kSub][tid], &cur_inst = s_lane[R::kInst][tid], &splitk = s_lane[R::kSplit][tid];
   PoolCtl *ctl = P.ctl;
 
   // ---- lane state -------------------------------------------------------
@@ -795,7 +804,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) 
       const uint4 *rec = reinterpret_cast<const uint4 *>(&P.subs[sub]);
       b0 = rec[0];
       b1 = rec[1];
-      cur_inst = MULTI ? b1.w | parity << 31 : b1.w;
+      if (MULTI) cur_inst = b1.w | parity << 31;
       const int limit = MULTI ? ld_volatile(&P.inst_limit[2 * b1.w + parity]) : P.inst_limit[b1.w];
       groot = (int)((b1.z >> 16) & 0xFFu);
       budget = limit - groot - 1;
@@ -1058,7 +1067,7 @@ __global__ void __launch_bounds__(BLOCK, threads_per_sm(W, PDB, MULTI) / BLOCK) 
       while (held) {
         const int src = (tid & ~31) + __ffs(held) - 1;
         held &= held - 1u;
-        const uint32_t first = s_lane[R::kCold + 3][src], hdr = s_lane[R::kCold + 5][src];
+        const uint32_t first = s_lane[R::kSub][src], hdr = s_lane[R::kSplit][src];
         const uint32_t n = hdr & 0xFFu;
         uint32_t t0 = 0;
         if (lane == 0) t0 = atomicAdd(&ctl->tail, n);
@@ -1427,7 +1436,7 @@ cudaError_t launch_split_level(int w, bool pdb, int num_sms, const SplitArgs &A,
 // Host launchers (template kernels stay in this translation unit).
 template <bool MULTI>
 static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, int num_sms, const RoundParams &P,
-                               cudaStream_t st, int *grid_out) {
+                               cudaStream_t st, int *lanes_out) {
   void (*kern)(RoundParams) = nullptr;
 #define SP_PICK(W, PD, B, WD) \
   if (w == W && pdb == PD && block == B) kern = search_round_kernel<W, PD, B, WD, MULTI>;
@@ -1440,6 +1449,11 @@ static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, in
   SP_PICK(5, false, 128, 10)
   SP_PICK(5, true, 128, 10)
 #undef SP_PICK
+  if (!MULTI && pdb && block == 256 && blocks_per_sm <= 0) {  // one block per SM
+    block = big_block(w);
+    kern = w == 4 ? search_round_kernel<4, true, big_block(4), 6, false>
+                  : search_round_kernel<5, true, big_block(5), 10, false>;
+  }
   if (!kern) return cudaErrorInvalidValue;
   int per_sm = blocks_per_sm;
   if (per_sm <= 0) {
@@ -1448,20 +1462,20 @@ static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, in
     if (per_sm < 1) per_sm = 1;
   }
   const int grid = num_sms * per_sm;
-  if (grid_out) *grid_out = grid;
+  if (lanes_out) *lanes_out = grid * block;
   kern<<<grid, block, 0, st>>>(P);
   note_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_search_round(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *grid_out) {
-  return launch_impl<false>(w, pdb, block, blocks_per_sm, num_sms, P, st, grid_out);
+                                const RoundParams &P, cudaStream_t st, int *lanes_out) {
+  return launch_impl<false>(w, pdb, block, blocks_per_sm, num_sms, P, st, lanes_out);
 }
 
 cudaError_t launch_search_multi(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *grid_out) {
-  return launch_impl<true>(w, pdb, block, blocks_per_sm, num_sms, P, st, grid_out);
+                                const RoundParams &P, cudaStream_t st, int *lanes_out) {
+  return launch_impl<true>(w, pdb, block, blocks_per_sm, num_sms, P, st, lanes_out);
 }
 
 cudaError_t launch_pool_init(Task *tasks, const uint32_t *n_emit, const uint32_t *direct, uint32_t n_direct,

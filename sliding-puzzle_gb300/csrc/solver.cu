@@ -811,7 +811,7 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
   P.reserve = s->cfg.donate_reserve < 0 ? 0u : s->cfg.donate_reserve > 0 ? (uint32_t)s->cfg.donate_reserve
                                                                           : lanes / 16u;
   P.spread = std::max(1u, lanes / 64u);  // lanes / 32 and / 16: 100 random 15-puzzles 1.4 and 2.5 % slower
-  int grid = 0;
+  int n_lanes = 0;
   if (multi) {
     MultiBufs &m = s->mb;
     P.inst_iter = m.iter;
@@ -838,10 +838,10 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
     P.handback_nodes = (unsigned long long)s->cfg.handback_nodes;
     P.sub_growth = m.use_growth ? m.growth : nullptr;
     SP_CUDA(s, launch_search_multi(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, P,
-                                   s->st, &grid));
+                                   s->st, &n_lanes));
   } else {
     SP_CUDA(s, launch_search_round(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, P,
-                                   s->st, &grid));
+                                   s->st, &n_lanes));
   }
   SP_CUDA(s, cudaEventRecord(s->ev1, s->st));
   SP_CUDA(s, s->h_ctl.reserve(1));
@@ -860,7 +860,7 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
   SP_CUDA(s, cudaEventElapsedTime(ms, s->ev0, s->ev1));
   s->stats.d2h_bytes += sizeof(PoolCtl) + 16 + n_subs * 8 + n_sol * sizeof(Solution);
   s->stats.kernel_launches += 2;
-  s->last_lanes = grid * block;
+  s->last_lanes = n_lanes;
   s->last_emitted = s->h_cnt.p[2];
   if (!s->h_ctl.p->error && s->h_cnt.p[3]) s->h_ctl.p->error = (int32_t)s->h_cnt.p[3];
   return SP_OK;
@@ -1833,10 +1833,10 @@ int sp_selftest_stall(sp_solver *s, int timeout_ms, int32_t *device_status) {
   P.poll_ns = SP_POLL_NS;
   P.reserve = 0;
   P.spread = 1;
-  int grid = 0;
+  int n_lanes = 0;
   const int block = s->cfg.threads_per_block == 128 ? 128 : 256;
   SP_CUDA(s, launch_search_round(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, P, s->st,
-                                 &grid));
+                                 &n_lanes));
   SP_CUDA(s, s->h_ctl.reserve(1));
   SP_CUDA(s, cudaMemcpyAsync(s->h_ctl.p, s->d_ctl, sizeof(PoolCtl), cudaMemcpyDeviceToHost, s->st));
   SP_CUDA(s, cudaStreamSynchronize(s->st));

@@ -65,10 +65,10 @@ constexpr int kGrowthSlacks = 8;
 
 // One threshold round: grid = num_sms * blocks_per_sm (0 = occupancy maximum).
 cudaError_t launch_search_round(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *grid_out);
+                                const RoundParams &P, cudaStream_t st, int *lanes_out);
 // The whole threshold loop of a batch in one launch (multi-iteration mode).
 cudaError_t launch_search_multi(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *grid_out);
+                                const RoundParams &P, cudaStream_t st, int *lanes_out);
 // Publish the round's tasks and reset the pool control block: the split
 // pieces (*n_emit of them, 0 when null), which the pre-pass has written to the
 // ring's first slots, then the direct tasks.
