@@ -428,12 +428,14 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
 // 24-puzzle, whose rows are longer, so that more threads leave it fewer shared
 // levels: 640 / 768 / 896 / 1024 65.3 / 63.8 / 70.3 / 72.7.
 // Blocks of 128 and 256 threads stay for a caller that asks for them or for a
-// number of blocks per SM.  Manhattan reads no tables: 768 or 1024 threads
-// measure alike.
+// number of blocks per SM.  Manhattan reads no tables and is bound by issue and
+// shared memory's latency: 1024 threads (blocks of 256, 768 an SM / one of 768
+// / 896 / 1024: 2048 24-puzzle roots 11.25 / 11.08 / 10.31 / 10.00 ms, 100
+// 15-puzzle walks 9.47 / 9.35 / 9.03 / 9.10).
 // The device loop is bound by its chains of small iterations, not by reads in
 // flight, and would spill 188 bytes at 64 registers: 768 threads (100 random
 // 15-puzzles 17.2 -> 17.0 ms).
-constexpr int big_block(int w) { return w == 4 ? 1024 : 768; }
+constexpr int big_block(int w, bool pdb) { return pdb && w == 5 ? 768 : 1024; }
 constexpr int shared_per_sm(int block) { return (block > 256 ? 164 : 192) * 1024; }
 constexpr int blocks_on_sm(int w, bool pdb, bool multi, int block) {
   return block > 256 ? 1 : (pdb && w == 4 && !multi ? 1024 : 768) / block;
@@ -1449,10 +1451,15 @@ static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, in
   SP_PICK(5, false, 128, 10)
   SP_PICK(5, true, 128, 10)
 #undef SP_PICK
-  if (!MULTI && pdb && block == 256 && blocks_per_sm <= 0) {  // one block per SM
-    block = big_block(w);
-    kern = w == 4 ? search_round_kernel<4, true, big_block(4), 6, false>
-                  : search_round_kernel<5, true, big_block(5), 10, false>;
+  if (!MULTI && block == 256 && blocks_per_sm <= 0) {  // one block per SM
+    block = big_block(w, pdb);
+    if (w == 4) {
+      kern = pdb ? search_round_kernel<4, true, big_block(4, true), 6, false>
+                 : search_round_kernel<4, false, big_block(4, false), 6, false>;
+    } else {
+      kern = pdb ? search_round_kernel<5, true, big_block(5, true), 10, false>
+                 : search_round_kernel<5, false, big_block(5, false), 10, false>;
+    }
   }
   if (!kern) return cudaErrorInvalidValue;
   int per_sm = blocks_per_sm;
