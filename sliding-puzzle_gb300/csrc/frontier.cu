@@ -6,15 +6,19 @@
 // src/24puzzle_block_parallel_with_pdb.cu:454-490).  Without pruning the
 // tree's shape -- which move sequences it holds, in breadth-first order --
 // depends only on the cell of the blank, so the host builds one template per
-// blank cell (moves from the root, parent, depth, children) and this kernel
-// applies it to every instance at once: one block per instance replays each
-// node's moves on the instance's board, computes h and the prefix maximum of
-// g + h along the node's path, and writes
+// blank cell (moves from the root, parent, depth, children) and two kernels
+// apply it to every instance at once: one replays each node's moves on the
+// instance's board and computes h, the other finds, a block per instance, the
+// prefix maximum of g + h along each node's path and writes
 //   * the leaves (depth D) as SubRoot records sorted by that maximum, ties in
 //     tree order (the active roots of a threshold round are then a prefix);
 //   * per maximum value: the number of leaves, the children generated by
 //     interior nodes, and the shallowest goal node (h == 0), which is what
 //     the threshold loop needs to count the nodes above the roots.
+// Bound by latency for one instance, on the path of every call: one 15-puzzle's
+// root set, with a block per instance for all of it and boards in local
+// memory, 84 us by Manhattan and 142 by tables (24-puzzles 205), now 55 and 58
+// (82), of which finding h takes 6 (26 for 50 24-puzzles).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -28,23 +32,100 @@ namespace {
 
 constexpr int kFrontThreads = 1024;
 constexpr int kFrontWarps = kFrontThreads / 32;
+constexpr int kHThreads = 256;  // of the kernel that finds h
 
-template <int W>
-__device__ __forceinline__ int replay(const uint8_t *root, int root_blank, uint64_t path, int depth, uint8_t *b) {
-  constexpr int N = W * W;
-  for (int c = 0; c < N; ++c) b[c] = root[c];
-  int blank = root_blank;
-  for (int j = 0; j < depth; ++j) {
-    const int d = (int)((path >> (2 * j)) & 3u);
-    const int src = blank + move_delta(W, d);
-    b[blank] = b[src];
-    b[src] = 0;
-    blank = src;
+// A thread's board: words of four cells, one column per thread ([word][thread]:
+// no bank conflict whatever cell a thread indexes; as byte arrays in local
+// memory, where the lanes of a warp hit up to 32 lines an access, the replays
+// took most of the kernel's time).
+template <int W, int T>
+struct BoardColumn {
+  static constexpr int kWords = (W * W + 3) / 4;
+  uint32_t *col;
+  __device__ __forceinline__ uint8_t &cell(int c) const {
+    return reinterpret_cast<uint8_t *>(col + (c >> 2) * T)[c & 3];
   }
-  return blank;
+  // the board after `depth` moves of `path` from the root; returns the blank's cell
+  __device__ __forceinline__ int replay(const uint32_t *root, int blank, uint64_t path, int depth) const {
+#pragma unroll
+    for (int q = 0; q < kWords; ++q) col[q * T] = root[q];
+    for (int j = 0; j < depth; ++j) {
+      const int src = blank + move_delta(W, (int)((path >> (2 * j)) & 3u));
+      cell(blank) = cell(src);
+      blank = src;
+    }
+    cell(blank) = 0;
+    return blank;
+  }
+};
+
+// The root's board as words, and its blank; the block synchronises afterwards.
+template <int W>
+__device__ __forceinline__ void load_root(const uint8_t *tiles, uint32_t (&s_root)[8], int &s_blank) {
+  if (threadIdx.x < 32) {
+    const uint8_t v = threadIdx.x < W * W ? tiles[threadIdx.x] : (uint8_t)0;
+    reinterpret_cast<uint8_t *>(s_root)[threadIdx.x] = v;
+    if (threadIdx.x < W * W && v == 0) s_blank = threadIdx.x;
+  }
 }
 
+// g + h of every node of every root set: `chunks` blocks per instance, so that
+// a single instance's 5000 nodes are spread over the SMs too.
 template <int W, bool PDB>
+__global__ void __launch_bounds__(kHThreads) frontier_h_kernel(FrontArgs A, uint32_t chunks) {
+  constexpr int N = W * W;
+  using Col = BoardColumn<W, kHThreads>;
+  __shared__ uint32_t s_root[8], s_board[Col::kWords][kHThreads];
+  __shared__ int s_blank;
+  const uint32_t li = blockIdx.x / chunks, ti = A.live_tmpl[li];
+  const FrontTmpl T = A.tmpl[ti];
+  const uint32_t first = (blockIdx.x % chunks) * kHThreads, x = first + threadIdx.x;
+  if (first >= T.n_nodes) return;
+  load_root<W>(A.tiles + (size_t)A.live[li] * N, s_root, s_blank);
+  __syncthreads();
+  if (x >= T.n_nodes) return;
+  const Col b{&s_board[0][threadIdx.x]};
+  const int dep = A.depth[T.node_off + x];
+  b.replay(s_root, s_blank, A.path[T.node_off + x], dep);
+  uint64_t ra = 0, rb = 0, fa = 0, fb = 0;
+  int h = 0;
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    const uint32_t t = (b.col[(c / 4) * kHThreads] >> (8 * (c % 4))) & 0xFFu;
+    if (PDB) {  // the packed index sums (HeurTables::sum)
+      const ulonglong2 *rec = reinterpret_cast<const ulonglong2 *>(A.ht->sum) + (t * N + c) * (W == 4 ? 1u : 2u);
+      const ulonglong2 v = __ldg(rec);
+      if (W == 4) {
+        ra += v.x;
+        fa += v.y;
+      } else {
+        const ulonglong2 u = __ldg(rec + 1);
+        ra += v.x;
+        rb += v.y;
+        fa += u.x;
+        fb += u.y;
+      }
+    } else if (t) {
+      h += abs(c / W - (int)t / W) + abs(c % W - (int)t % W);
+    }
+  }
+  if (PDB) {
+    constexpr int kPat = W == 4 ? 3 : 4;
+    int hr = 0, hf = 0;
+#pragma unroll
+    for (int p = 0; p < kPat; ++p) {
+      const uint32_t base = W == 4 ? (uint32_t)p << 20 : (p ? 1u << 28 : 0u);
+      hr += __ldg(A.pdb + (sum_field<W>(ra, rb, p) | base));
+      hf += __ldg(A.pdb + (sum_field<W>(fa, fb, p) | base));
+    }
+    h = max(hr, hf);
+  }
+  A.f[A.live_scratch[li] + x] = (int16_t)(dep + h);
+}
+
+// The rest of an instance's root set, a block each: prefix maxima, sums and
+// the sorted leaves.
+template <int W>
 __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A) {
   constexpr int N = W * W;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -57,19 +138,16 @@ __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A) {
   const int32_t *parent = A.parent + T.node_off;
   const uint8_t *nchild = A.nchild + T.node_off;
   const uint8_t *depth = A.depth + T.node_off;
-  int16_t *F = A.f + A.live_scratch[li];
+  const int16_t *F = A.f + A.live_scratch[li];
   int16_t *M = A.maxf + A.live_scratch[li];
 
-  __shared__ uint8_t s_root[32];
+  using Col = BoardColumn<W, kFrontThreads>;
+  __shared__ uint32_t s_root[8], s_board[Col::kWords][kFrontThreads];
   __shared__ int s_blank, s_bad;
   __shared__ uint32_t s_leaf[kFrontBuckets], s_child[kFrontBuckets], s_goal[kFrontBuckets];
   __shared__ uint32_t s_wcnt[kFrontWarps][kFrontBuckets];
 
-  if (tid < N) {
-    const uint8_t v = A.tiles[(size_t)inst * N + tid];
-    s_root[tid] = v;
-    if (v == 0) s_blank = tid;
-  }
+  load_root<W>(A.tiles + (size_t)inst * N, s_root, s_blank);
   for (int b = tid; b < kFrontBuckets; b += kFrontThreads) {
     s_leaf[b] = 0;
     s_child[b] = 0;
@@ -79,14 +157,7 @@ __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A) {
   if (tid == 0) s_bad = 0;
   __syncthreads();
 
-  // 1. g + h of every node
-  uint8_t bd[N];
-  for (uint32_t x = tid; x < T.n_nodes; x += kFrontThreads) {
-    const int dep = depth[x];
-    replay<W>(s_root, s_blank, path[x], dep, bd);
-    F[x] = (int16_t)(dep + board_h<W, PDB>(bd, A.ht, A.pdb));
-  }
-  __syncthreads();
+  // 1. (frontier_h_kernel) g + h of every node
   const int h0 = F[0];
   // 2. prefix maximum of g + h along each path, one level at a time (the
   //    parent of a level-d node is on level d - 1)
@@ -112,12 +183,21 @@ __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A) {
     if (tid == 0) atomicCAS(A.error, 0, (int32_t)SP_ERR_ARG);
     return;
   }
-  if (tid == 0) {  // exclusive prefix of the leaf counts, kept in s_leaf
-    uint32_t c = 0;
-    for (int b = 0; b < kFrontBuckets; ++b) {
-      const uint32_t v = s_leaf[b];
-      s_leaf[b] = c;
-      c += v;
+  if (warp == 0) {  // exclusive prefix of the leaf counts, kept in s_leaf
+    constexpr int kEach = kFrontBuckets / 32;
+    uint32_t v[kEach], sum = 0;
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) sum += v[q] = s_leaf[lane * kEach + q];
+    uint32_t c = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, c, o);
+      if (lane >= o) c += u;
+    }
+    c -= sum;
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+      s_leaf[lane * kEach + q] = c;
+      c += v[q];
     }
   }
   __syncthreads();
@@ -138,17 +218,14 @@ __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A) {
       uint32_t pos = s_leaf[b] + rank;
       for (int q = 0; q < warp; ++q) pos += s_wcnt[q][b];
       const uint32_t j = base + pos;
-      SubRoot r{};
-      const int blank = replay<W>(s_root, s_blank, path[x], (int)T.D, bd);
-      for (int c = 0; c < N; ++c) r.board[c] = bd[c];
-      r.blank = (uint8_t)blank;
-      r.g = (uint8_t)T.D;
-      r.pre = T.D ? (uint8_t)((path[x] >> (2 * (T.D - 1))) & 3u) : kNoPre;
-      r.inst = inst;
-      const uint4 *src = reinterpret_cast<const uint4 *>(&r);
+      const Col bd{&s_board[0][tid]};
+      const int blank = bd.replay(s_root, s_blank, path[x], (int)T.D);
+      const uint32_t pre = T.D ? (uint32_t)(path[x] >> (2 * (T.D - 1))) & 3u : kNoPre;
+      const uint32_t tail = (uint32_t)blank << 8 | T.D << 16 | pre << 24;
+      auto word = [&](int q) -> uint32_t { return q < Col::kWords ? bd.col[q * kFrontThreads] : 0u; };
       uint4 *dst = reinterpret_cast<uint4 *>(A.subs + j);
-      dst[0] = src[0];
-      dst[1] = src[1];
+      dst[0] = make_uint4(word(0), word(1), word(2), word(3));
+      dst[1] = make_uint4(word(4), word(5), (word(6) & 0xFFu) | tail, inst);
       A.leaf_maxf[j] = M[x];
       A.leaf_h[j] = (uint8_t)(F[x] - (int)T.D);
       A.leaf_node[j] = (int32_t)x;
@@ -179,16 +256,21 @@ __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A) {
 
 }  // namespace
 
-cudaError_t launch_frontier(int w, bool pdb, int n_live, const FrontArgs &A, cudaStream_t st) {
+cudaError_t launch_frontier(int w, bool pdb, int n_live, uint32_t max_nodes, const FrontArgs &A, cudaStream_t st) {
   if (n_live <= 0) return cudaSuccess;
+  const uint32_t chunks = (max_nodes + kHThreads - 1) / kHThreads;
+  const uint64_t grid = (uint64_t)n_live * chunks;
+  if (!chunks || grid > 0x7FFFFFFFull) return cudaErrorInvalidConfiguration;
   if (w == 4) {
-    if (pdb) frontier_kernel<4, true><<<n_live, kFrontThreads, 0, st>>>(A);
-    else frontier_kernel<4, false><<<n_live, kFrontThreads, 0, st>>>(A);
+    if (pdb) frontier_h_kernel<4, true><<<(uint32_t)grid, kHThreads, 0, st>>>(A, chunks);
+    else frontier_h_kernel<4, false><<<(uint32_t)grid, kHThreads, 0, st>>>(A, chunks);
+    frontier_kernel<4><<<n_live, kFrontThreads, 0, st>>>(A);
   } else {
-    if (pdb) frontier_kernel<5, true><<<n_live, kFrontThreads, 0, st>>>(A);
-    else frontier_kernel<5, false><<<n_live, kFrontThreads, 0, st>>>(A);
+    if (pdb) frontier_h_kernel<5, true><<<(uint32_t)grid, kHThreads, 0, st>>>(A, chunks);
+    else frontier_h_kernel<5, false><<<(uint32_t)grid, kHThreads, 0, st>>>(A, chunks);
+    frontier_kernel<5><<<n_live, kFrontThreads, 0, st>>>(A);
   }
-  note_launch();
+  note_launch(2);
   return cudaGetLastError();
 }
 

@@ -90,14 +90,6 @@ __device__ __forceinline__ unsigned long long globaltimer() {
   return t;
 }
 
-// Field p of packed pattern indices (HeurTables::sum): width 4 three 20-bit
-// fields in one word, width 5 four 28-bit fields, two to a word.
-template <int W>
-__device__ __forceinline__ uint32_t sum_field(uint64_t a, uint64_t b, int p) {
-  if (W == 4) return (uint32_t)(a >> (20 * p)) & 0xFFFFFu;
-  return (uint32_t)((p >> 1 ? b : a) >> (28 * (p & 1))) & 0xFFFFFFFu;
-}
-
 // Blank displacement of move d without compares: the four displacements as
 // signed bytes of one immediate, byte d sign-extended by one permute.
 template <int W>

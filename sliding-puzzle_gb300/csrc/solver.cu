@@ -524,7 +524,7 @@ int build_root_sets(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &i
   }
   // per live instance: template, first SubRoot, first scratch node
   const size_t nl = live.size();
-  size_t n_subs = 0, n_nodes = 0;
+  size_t n_subs = 0, n_nodes = 0, max_nodes = 0;
   std::vector<uint32_t> arr(4 * std::max<size_t>(nl, 1), 0);
   for (size_t k = 0; k < nl; ++k) {
     Instance &I = inst[live[k]];
@@ -537,6 +537,7 @@ int build_root_sets(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &i
     arr[3 * nl + k] = (uint32_t)n_nodes;
     n_subs += I.n_leaves;
     n_nodes += T.path.size();
+    max_nodes = std::max(max_nodes, T.path.size());
   }
   *n_subs_out = n_subs;
   if ((rc = ensure(s, &s->d_subs, &s->subs_cap, std::max<size_t>(n_subs, 1))) ||
@@ -587,8 +588,8 @@ int build_root_sets(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &i
   A.leaf_node = fb.leaf_node;
   A.out = fb.out;
   A.error = fb.error;
-  SP_CUDA(s, launch_frontier(w, s->heur == SP_HEUR_PDB, (int)nl, A, s->st));
-  s->stats.kernel_launches += 1;
+  SP_CUDA(s, launch_frontier(w, s->heur == SP_HEUR_PDB, (int)nl, (uint32_t)max_nodes, A, s->st));
+  s->stats.kernel_launches += 2;
   SP_CUDA(s, cudaMemcpyAsync(fb.h_out.p, fb.out, nl * sizeof(FrontInst), cudaMemcpyDeviceToHost, s->st));
   SP_CUDA(s, cudaMemcpyAsync(fb.h_error.p, fb.error, sizeof(int32_t), cudaMemcpyDeviceToHost, s->st));
   SP_CUDA(s, cudaStreamSynchronize(s->st));

@@ -6,6 +6,14 @@
 
 namespace sp {
 
+// Field p of packed pattern indices (HeurTables::sum): width 4 three 20-bit
+// fields in one word, width 5 four 28-bit fields, two to a word.
+template <int W>
+__device__ __forceinline__ uint32_t sum_field(uint64_t a, uint64_t b, int p) {
+  if (W == 4) return (uint32_t)(a >> (20 * p)) & 0xFFFFFu;
+  return (uint32_t)((p >> 1 ? b : a) >> (28 * (p & 1))) & 0xFFFFFFFu;
+}
+
 // Heuristic of a board from scratch: Manhattan distance, or the additive PDB
 // value max(sum of regular-partition lookups, sum of reflected lookups) with
 // tables at t << 20 (width 4) or t << 28 (width 5) in `tables`.

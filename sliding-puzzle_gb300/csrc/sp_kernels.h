@@ -142,7 +142,8 @@ struct FrontArgs {
   FrontInst *out;                // [block]
   int32_t *error;
 };
-cudaError_t launch_frontier(int w, bool pdb, int n_live, const FrontArgs &A, cudaStream_t st);
+// max_nodes: the largest of the templates in use.
+cudaError_t launch_frontier(int w, bool pdb, int n_live, uint32_t max_nodes, const FrontArgs &A, cudaStream_t st);
 
 // h of n boards (n * N bytes) into h[n]; PDB tables as in RoundParams.
 cudaError_t launch_heuristic(int w, bool pdb, const uint8_t *boards, int n, int32_t *h,
