@@ -130,21 +130,31 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
-int check_instance(int w, const uint8_t *t) {
-  const int n = w * w;
+bool is_permutation(int n, const uint8_t *t) {
   uint32_t seen = 0;
   for (int i = 0; i < n; ++i) {
-    if (t[i] >= n || ((seen >> t[i]) & 1u)) return SP_ERR_NOT_PERMUTATION;
+    if (t[i] >= n) return false;
     seen |= 1u << t[i];
   }
-  int inv = 0, brow = 0;
-  for (int i = 0; i < n; ++i) {
-    if (!t[i]) { brow = i / w; continue; }
-    for (int j = i + 1; j < n; ++j)
-      if (t[j] && t[j] < t[i]) ++inv;
-  }
+  return seen == (1u << n) - 1u;
+}
+
+int check_instance(int w, const uint8_t *t) {
+  const int n = w * w;
+  if (!is_permutation(n, t)) return SP_ERR_NOT_PERMUTATION;
+  // parity of the inversions among the tiles: the permutation's (its length
+  // less its cycles) without the blank's inversions, one with every cell
+  // before it
+  uint32_t left = (1u << n) - 1u;
+  int cycles = 0, blank = 0;
+  for (; left; ++cycles)
+    for (int i = __builtin_ctz(left); (left >> i) & 1u; i = t[i]) {
+      left &= ~(1u << i);
+      if (!t[i]) blank = i;
+    }
   // goal blank at cell 0: odd widths keep inversion parity; even widths keep
   // inversions + blank row
+  const int inv = n - cycles + blank, brow = blank / w;
   const int par = (w & 1) ? (inv & 1) : ((inv + brow) & 1);
   return par ? SP_ERR_UNSOLVABLE : SP_OK;
 }
@@ -1693,14 +1703,8 @@ int sp_root_set_template(int width, int blank, int target, uint64_t *paths, uint
   return SP_OK;
 }
 
-int sp_heuristic(sp_solver *s, const uint8_t *tiles, int n, int32_t *h) {
-  if (!s || (n > 0 && (!tiles || !h)) || n < 0) return SP_ERR_ARG;
-  if (s->heur == SP_HEUR_PDB && !s->pdb_ready) return SP_ERR_NO_PDB;
-  if (n == 0) return SP_OK;
-  for (int i = 0; i < n; ++i) {
-    const int st = check_instance(s->w, tiles + (size_t)i * s->n);
-    if (st == SP_ERR_NOT_PERMUTATION) return st;
-  }
+// h of n > 0 boards that have been checked.
+static int heuristic_rows(sp_solver *s, const uint8_t *tiles, int n, int32_t *h) {
   int rc = ensure(s, &s->d_boards, &s->boards_cap, (size_t)n * s->n);
   if (rc) return rc;
   rc = ensure(s, &s->d_h, &s->h_cap, (size_t)n);
@@ -1712,6 +1716,15 @@ int sp_heuristic(sp_solver *s, const uint8_t *tiles, int n, int32_t *h) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
   if (e != cudaSuccess) return fail_cuda(s, e, "sp_heuristic");
   return SP_OK;
+}
+
+int sp_heuristic(sp_solver *s, const uint8_t *tiles, int n, int32_t *h) {
+  if (!s || (n > 0 && (!tiles || !h)) || n < 0) return SP_ERR_ARG;
+  if (s->heur == SP_HEUR_PDB && !s->pdb_ready) return SP_ERR_NO_PDB;
+  if (n == 0) return SP_OK;
+  for (int i = 0; i < n; ++i)
+    if (!is_permutation(s->n, tiles + (size_t)i * s->n)) return SP_ERR_NOT_PERMUTATION;
+  return heuristic_rows(s, tiles, n, h);
 }
 
 int sp_solve_batch(sp_solver *s, const uint8_t *tiles, int n, sp_result *results) {
@@ -1743,7 +1756,7 @@ int sp_dfs_round(sp_solver *s, const uint8_t *roots, const int32_t *depth, const
   plan.direct.resize((size_t)n);
   for (int i = 0; i < n; ++i) {
     const uint8_t *t = roots + (size_t)i * s->n;
-    if (check_instance(s->w, t) == SP_ERR_NOT_PERMUTATION) return SP_ERR_NOT_PERMUTATION;
+    if (!is_permutation(s->n, t)) return SP_ERR_NOT_PERMUTATION;
     if (depth[i] < 0 || depth[i] > 255 || pre[i] < -1 || pre[i] > 3) return SP_ERR_ARG;
     SubRoot r{};
     memcpy(r.board, t, (size_t)s->n);
@@ -1758,7 +1771,7 @@ int sp_dfs_round(sp_solver *s, const uint8_t *roots, const int32_t *depth, const
   // roots that are goals (the reference's dfs_kernel sets dev_flag for them,
   // src/24puzzle_block_parallel_with_pdb.cu:580-583)
   std::vector<int32_t> h((size_t)n);
-  int rc = sp_heuristic(s, roots, n, h.data());
+  int rc = heuristic_rows(s, roots, n, h.data());
   if (rc) return rc;
   for (int i = 0; i < n; ++i)
     if (h[(size_t)i] == 0 && (*found < 0 || depth[i] < *found)) *found = depth[i];
