@@ -242,7 +242,7 @@ extern "C" int sp_dfs_round_md_noalloc(int width, const uint8_t *d_roots, const 
     P.steps = 32;
     P.donate = 1;
     P.timeout_ns = 20000000000ull;
-    P.poll_ns = 2000;
+    P.poll_ns = 4000;
     const uint32_t lanes = (uint32_t)num_sms * 1024u;
     P.reserve = lanes / 16u;
     P.spread = lanes / 64u;

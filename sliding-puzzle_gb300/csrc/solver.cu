@@ -75,9 +75,11 @@
 #endif
 
 // Shortest interval between two reads of the pool's control words by one
-// block (ns); the block shares what it read.
+// block (ns); the block shares what it read (1000 / 2000 / 4000 / 8000: 100
+// random 15-puzzles 16.4 / 16.1 / 15.85 / 15.8 ms, one walk of 40 moves 0.47 /
+// 0.475 / 0.463 / 0.47).
 #ifndef SP_POLL_NS
-#define SP_POLL_NS 2000
+#define SP_POLL_NS 4000
 #endif
 
 namespace sp {
