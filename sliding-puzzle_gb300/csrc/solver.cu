@@ -567,7 +567,7 @@ int build_root_sets(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &i
       (rc = ensure(s, &fb.leaf_maxf, &fb.cap_leaf_maxf, n_subs)) ||
       (rc = ensure(s, &fb.leaf_node, &fb.cap_leaf_node, n_subs)) ||
       (rc = ensure(s, &fb.leaf_h, &fb.cap_leaf_h, n_subs)) || (rc = ensure(s, &fb.out, &fb.cap_out, nl)) ||
-      (rc = ensure(s, &fb.error, &fb.cap_error, (size_t)1)))
+      (rc = ensure(s, &fb.error, &fb.cap_error, 1 + nl)))
     return rc;
   SP_CUDA(s, fb.h_in.reserve(in_bytes));
   SP_CUDA(s, fb.h_out.reserve(nl));
@@ -575,7 +575,7 @@ int build_root_sets(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &i
   memcpy(fb.h_in.p, tiles, inst.size() * (size_t)n);
   memcpy(fb.h_in.p + tiles_bytes, arr.data(), 4 * nl * sizeof(uint32_t));
   SP_CUDA(s, cudaMemcpyAsync(fb.in, fb.h_in.p, in_bytes, cudaMemcpyHostToDevice, s->st));
-  SP_CUDA(s, cudaMemsetAsync(fb.error, 0, sizeof(int32_t), s->st));
+  SP_CUDA(s, cudaMemsetAsync(fb.error, 0, (1 + nl) * sizeof(int32_t), s->st));
   s->stats.h2d_bytes += in_bytes;
   const uint32_t *d_arr = reinterpret_cast<const uint32_t *>(fb.in + tiles_bytes);
   FrontArgs A{};
@@ -600,8 +600,9 @@ int build_root_sets(sp_solver *s, const uint8_t *tiles, std::vector<Instance> &i
   A.leaf_node = fb.leaf_node;
   A.out = fb.out;
   A.error = fb.error;
+  A.arrived = reinterpret_cast<uint32_t *>(fb.error + 1);
   SP_CUDA(s, launch_frontier(w, s->heur == SP_HEUR_PDB, (int)nl, (uint32_t)max_nodes, A, s->st));
-  s->stats.kernel_launches += 2;
+  s->stats.kernel_launches += 1;
   SP_CUDA(s, cudaMemcpyAsync(fb.h_out.p, fb.out, nl * sizeof(FrontInst), cudaMemcpyDeviceToHost, s->st));
   SP_CUDA(s, cudaMemcpyAsync(fb.h_error.p, fb.error, sizeof(int32_t), cudaMemcpyDeviceToHost, s->st));
   SP_CUDA(s, cudaStreamSynchronize(s->st));

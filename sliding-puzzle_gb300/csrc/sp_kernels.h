@@ -135,6 +135,7 @@ struct FrontArgs {
   const HeurTables *ht;
   const uint8_t *pdb;
   int16_t *f, *maxf;             // scratch, one entry per node
+  uint32_t *arrived;             // [live instance] blocks that have finished h, 0 at the start
   SubRoot *subs;                 // leaves, sorted by maxf per instance
   int32_t *leaf_maxf;
   uint8_t *leaf_h;
