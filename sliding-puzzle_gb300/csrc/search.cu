@@ -26,10 +26,12 @@
 //    one tile into the blank), without a branch between the two.
 //    Bound by issue and by table reads in flight.  Against the version with
 //    register boards and indices, whose lanes drifted apart (9-15 of 32
-//    active per instruction, 18-21 warp instructions per node; now 18 and
-//    10): 100 random 15-puzzles 28.8 -> 19.7 ms, 4096 mixed ones 348 -> 211
-//    ms (70 -> 116 G nodes/s), 100 Manhattan walks 29.2 -> 18.9 ms, 16384
-//    24-puzzle roots 166 -> 101 ms;
+//    active per instruction, 18-21 warp instructions per node), this step
+//    alone, then with the choices of donors, block and L1 described below (21-24
+//    and 5-9): 100 random 15-puzzles 28.8 -> 19.7 -> 15.9 ms, 4096 mixed ones
+//    348 -> 211 -> 156 ms (the large rounds 70 -> 116 -> 140 G nodes/s), 100
+//    Manhattan walks 29.2 -> 18.9 -> 8.9 ms, 16384 24-puzzle roots 166 -> 101
+//    -> 59 ms;
 //  * load balance by a device task pool: lanes claim slots warp-aggregated
 //    (ballot + one atomicAdd per warp); claims may run ahead of the pool's
 //    tail, and while any lane waits, busy lanes donate the untried moves of
