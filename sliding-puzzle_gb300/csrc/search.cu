@@ -485,7 +485,7 @@ struct WarpState {
 static_assert(sizeof(WarpState) == 64, "WarpState layout");
 
 template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
-__global__ void __launch_bounds__(BLOCK, blocks_on_sm(W, PDB, MULTI, BLOCK)) search_round_kernel(RoundParams P) {
+__device__ __forceinline__ void search_round(const RoundParams &P) {
   using R = LaneRows<W, PDB, BLOCK, WORDS, MULTI>;
   constexpr int N = W * W;
   constexpr unsigned FULL = 0xffffffffu;
@@ -1244,6 +1244,17 @@ __global__ void __launch_bounds__(BLOCK, blocks_on_sm(W, PDB, MULTI, BLOCK)) sea
   if (tid < 5) atomicAdd(&ctl->counters[4 + tid], (unsigned long long)s_stat[tid]);
 }
 
+template <int W, bool PDB, int BLOCK, int WORDS, bool MULTI>
+__global__ void __launch_bounds__(BLOCK, blocks_on_sm(W, PDB, MULTI, BLOCK)) search_round_kernel(RoundParams P) {
+  search_round<W, PDB, BLOCK, WORDS, MULTI>(P);
+}
+
+// A round in one block per SM.
+template <int W, bool PDB>
+__global__ void __launch_bounds__(big_block(W, PDB), 1) search_sm_kernel(RoundParams P) {
+  search_round<W, PDB, big_block(W, PDB), W == 4 ? 6 : 10, false>(P);
+}
+
 // Reset the ring (seq[s] = s: slot s free for index s) and publish the round's
 // tasks at indices [0, n) (seq = index + 1): the pieces of split roots first,
 // which the pre-pass has left in their slots, then the host's direct tasks
@@ -1447,13 +1458,8 @@ static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, in
 #undef SP_PICK
   if (!MULTI && block == 256 && blocks_per_sm <= 0) {  // one block per SM
     block = big_block(w, pdb);
-    if (w == 4) {
-      kern = pdb ? search_round_kernel<4, true, big_block(4, true), 6, false>
-                 : search_round_kernel<4, false, big_block(4, false), 6, false>;
-    } else {
-      kern = pdb ? search_round_kernel<5, true, big_block(5, true), 10, false>
-                 : search_round_kernel<5, false, big_block(5, false), 10, false>;
-    }
+    if (w == 4) kern = pdb ? search_sm_kernel<4, true> : search_sm_kernel<4, false>;
+    else kern = pdb ? search_sm_kernel<5, true> : search_sm_kernel<5, false>;
   }
   if (!kern) return cudaErrorInvalidValue;
   int per_sm = blocks_per_sm;
