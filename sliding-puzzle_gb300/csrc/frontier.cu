@@ -68,7 +68,7 @@ __device__ __forceinline__ void load_root(const uint8_t *tiles, uint32_t (&s_roo
   }
 }
 
-// `chunks` blocks per instance, so that a single instance's 5000 nodes are
+// `chunks` blocks per instance, so that a single instance's 11400 nodes are
 // spread over SMs too; the one that finishes last does the rest.
 template <int W, bool PDB>
 __global__ void __launch_bounds__(kFrontThreads) frontier_kernel(FrontArgs A, uint32_t chunks) {
