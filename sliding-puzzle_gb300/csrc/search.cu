@@ -577,7 +577,7 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
   int krare = 0;                 // entering a child of a level from here on needs a second look: the
                                  // first level of a split task, levels beyond the shared ones or the
                                  // last that the lane's stack and path can hold
-  int groot = 0, plen = 0;
+  int plen = 0;
   int lo = 0;                    // donation: no level below lo has untried moves
   int lo_slack = 0;              // the limit less f at level lo (kHarder)
   uint32_t cnt = 0;              // generated nodes not yet added to the task's counters
@@ -658,7 +658,7 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     }
     const int len = plen + level;
     wb[25] = (uint8_t)at;
-    wb[26] = (uint8_t)(groot + level);
+    wb[26] = 0;
     wb[27] = (uint8_t)mask;
     w[7] = sub;
     Task *D = &P.tasks[t & (P.cap - 1u)];
@@ -802,12 +802,10 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
       b1 = rec[1];
       if (MULTI) cur_inst = b1.w | parity << 31;
       const int limit = MULTI ? ld_volatile(&P.inst_limit[2 * b1.w + parity]) : P.inst_limit[b1.w];
-      groot = (int)((b1.z >> 16) & 0xFFu);
-      budget = limit - groot - 1;
+      budget = limit - (int)((b1.z >> 16) & 0xFFu) - 1;
       pre = (b1.z >> 24) == kNoPre ? -1 : (int)(b1.z >> 24);
     } else {
       if (MULTI) cur_inst = P.subs[sub].inst | parity << 31;
-      groot = (int)((b1.z >> 16) & 0xFFu);
       budget = (int)meta >> 16;
     }
     blank = (int)((b1.z >> 8) & 0xFFu);
@@ -823,7 +821,7 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     if (W == 5) {
       me[(R::kBoard + 4) * BLOCK] = start_board[4] = b1.x;
       me[(R::kBoard + 5) * BLOCK] = start_board[5] = b1.y;
-      me[(R::kBoard + 6) * BLOCK] = b1.z;  // cell 24, then the record's blank and g
+      me[(R::kBoard + 6) * BLOCK] = b1.z;  // cell 24, then the record's blank
     }
     start_board[6] = b1.z;
     boff = board_off(blank);
@@ -836,11 +834,14 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     return h <= budget + 1;
   };
   auto record_goal = [&]() {
-    const uint32_t si = P.subs[sub].inst;
+    const SubRoot *root = &P.subs[sub];
+    const uint32_t si = root->inst;
     Solution *S = &P.sol[MULTI ? 2 * si + (cur_inst >> 31) : si];
-    atomicMax(&S->best, 0xFFFFFFFFu - (uint32_t)(groot + k));  // shortest goal depth over all lanes
+    const int len = plen + k;
+    // shortest goal depth over all lanes; from the root's depth, which may be
+    // up to 255, so that no record between holds a depth in a byte
+    atomicMax(&S->best, 0xFFFFFFFFu - ((uint32_t)root->g + (uint32_t)len));
     if (atomicCAS(&S->flag, 0u, 1u) == 0u) {
-      int len = plen + k;
       S->sub = sub;
       S->len = (uint32_t)len;
       write_path(len, [&](int wi, uint32_t w) { S->path[wi] = w; });
@@ -1389,10 +1390,10 @@ __global__ void __launch_bounds__(128) split_level_kernel(SplitArgs A) {
       }
       return v;
     };
-    const uint32_t g = (b1.z >> 16) & 0xFFu;
     if (keep && h == 0) {  // a goal at the child: record it like the search does
-      Solution *S = &A.sol[A.subs[sub].inst];
-      atomicMax(&S->best, 0xFFFFFFFFu - (g + 1u));
+      const SubRoot *root = &A.subs[sub];
+      Solution *S = &A.sol[root->inst];
+      atomicMax(&S->best, 0xFFFFFFFFu - ((uint32_t)root->g + (uint32_t)plen + 1u));
       if (atomicCAS(&S->flag, 0u, 1u) == 0u) {
         S->sub = sub;
         S->len = (uint32_t)(plen + 1);
@@ -1419,7 +1420,7 @@ __global__ void __launch_bounds__(128) split_level_kernel(SplitArgs A) {
       uint4 *out = reinterpret_cast<uint4 *>(dst);
       const uint32_t child = step_legal<W>(src) & ~(1u << (3 - d));
       out[0] = make_uint4(nw[0], nw[1], nw[2], nw[3]);
-      out[1] = make_uint4(nw[4], nw[5], (nw[6] & 0xFFu) | (uint32_t)src << 8 | (g + 1u) << 16 | child << 24, sub);
+      out[1] = make_uint4(nw[4], nw[5], (nw[6] & 0xFFu) | (uint32_t)src << 8 | child << 24, sub);
       *reinterpret_cast<uint32_t *>(out + 2) =
           (uint32_t)(plen + 1) | (levels - 1u) << 8 | (uint32_t)min(budget - 1, kMaxBudget) << 16;
       for (int q = 0; 16 * q <= plen; ++q) dst->path[q] = child_path(q);

@@ -98,10 +98,11 @@ static_assert(sizeof(SubRoot) == 32, "SubRoot layout");
 // Unit of work in the device task pool: the node reached from SubRoot `sub`
 // by `plen` moves, restricted to the first-level moves in `mask`.  A task
 // below its root (plen > 0) carries its board, so that its claimant need not
-// replay the path; of a root itself only mask, sub, plen and flags count.
+// replay the path; its depth is its SubRoot's plus plen.  Of a root itself only
+// mask, sub, plen and flags count.
 struct alignas(16) Task {
   uint8_t board[kMaxN];
-  uint8_t blank, g;
+  uint8_t blank, pad0;
   uint8_t mask;     // plen > 0: legal moves only, none of them the reverse
   uint32_t sub;
   uint8_t plen;
