@@ -526,6 +526,7 @@ __global__ void __launch_bounds__(kEmbThreads, 1) embed_kernel(EmbedArgs A) {
         acc[q].w += v.w;
       }
     }
+    __syncwarp();  // all lanes have read the rows' features: the next tile overwrites them
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       __nv_bfloat162 h[2];
