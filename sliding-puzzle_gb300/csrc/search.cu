@@ -801,7 +801,9 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
       b0 = rec[0];
       b1 = rec[1];
       if (MULTI) cur_inst = b1.w | parity << 31;
-      const int limit = MULTI ? ld_volatile(&P.inst_limit[2 * b1.w + parity]) : P.inst_limit[b1.w];
+      // below 0 no root is entered, whatever its g and h; a caller's limit of
+      // INT_MIN less g would wrap
+      const int limit = max(MULTI ? ld_volatile(&P.inst_limit[2 * b1.w + parity]) : P.inst_limit[b1.w], -1);
       budget = limit - (int)((b1.z >> 16) & 0xFFu) - 1;
       pre = (b1.z >> 24) == kNoPre ? -1 : (int)(b1.z >> 24);
     } else {
