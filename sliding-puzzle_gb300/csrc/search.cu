@@ -764,7 +764,8 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
       __threadfence();
     }
     // one launch, one threshold: the counts are read after the kernel, so no
-    // fence; the tasks this one gave away were counted before (below)
+    // fence; the tasks this one gave away were counted before, by this lane or
+    // ahead of the warp barrier in the donation below
     atomicSub(&ctl->outstanding, 1u);
   };
   // Copy the claimed record out of its ring slot, free the slot for the
@@ -1206,12 +1207,15 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
       uint32_t tbase = 0;
       const int lead = donors ? __ffs(donors) - 1 : 0;
       if (donors && lane == lead) {
-        const uint32_t before = atomicAdd(&ctl->outstanding, (uint32_t)__popc(donors));
+        atomicAdd(&ctl->outstanding, (uint32_t)__popc(donors));
         tbase = atomicAdd(&ctl->tail, (uint32_t)__popc(donors));
-        // counted as outstanding before any donor can finish its own task
-        asm volatile("" ::"r"(before) : "memory");
       }
       tbase = __shfl_sync(FULL, tbase, lead);
+      // The lead lane's count comes before what any donor, or the claimant of
+      // what it publishes, takes off again, so that `outstanding` never reads 0
+      // while work is left: a warp barrier orders memory among the warp's lanes
+      // (a shuffle does not), a record's release and acquire the rest.
+      __syncwarp();
       if (donor) {
         // the reserved index's ring slot is free once the slot's previous
         // occupant (index t - cap, claimed long before) was copied out, which
