@@ -73,7 +73,7 @@ typedef enum {
 typedef struct {
   int32_t frontier_target;   /* subproblems per instance (default 3072; the
                                 reference's BLOCK_NUM is 2048);
-                                a batch is capped near 8 per resident GPU lane
+                                a batch is capped near 8 per lane of a round
                                 (at least 32 per instance) */
   int32_t threads_per_block; /* 128 or 256 */
   int32_t blocks_per_sm;     /* 0 = occupancy maximum */

@@ -243,11 +243,11 @@ extern "C" int sp_dfs_round_md_noalloc(int width, const uint8_t *d_roots, const 
     P.donate = 1;
     P.timeout_ns = 20000000000ull;
     P.poll_ns = 4000;
-    const uint32_t lanes = (uint32_t)num_sms * 1024u;
+    uint32_t lanes = 0;
+    if (search_lanes(width, false, 256, 0, num_sms, false, &lanes) != cudaSuccess) return SP_ERR_CUDA;
     P.reserve = lanes / 16u;
     P.spread = lanes / 64u;
-    int lanes_run = 0;
-    if (launch_search_round(width, false, 256, 0, num_sms, P, st, &lanes_run) != cudaSuccess) return SP_ERR_CUDA;
+    if (launch_search(width, false, 256, 0, num_sms, false, P, st) != cudaSuccess) return SP_ERR_CUDA;
   }
   noalloc_finish_kernel<<<1, 1, 0, st>>>(base, d_found);
   if (!launched(1)) return SP_ERR_CUDA;

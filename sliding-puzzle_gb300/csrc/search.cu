@@ -1126,11 +1126,14 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     // next iteration waits for the last one's tasks (32 / 40 / 48 steps: 100
     // random 15-puzzles 17.4 / 16.9 / 16.9 ms, 2048 24-puzzle roots 11.8 / 11.3
     // / 11.2, 50 24-puzzles 12.7 / 12.9 / 12.9).
-    // While three lanes in four wait, they are half as long: issue slots are
-    // free and what counts is how fast work spreads (32 / 16 / 8 steps then: 50
-    // 24-puzzles 12.8 / 12.3 / 12.6, one random 15-puzzle 1.60 / 1.52 / 1.51,
-    // 100 Manhattan walks 9.41 / 9.42 / 9.58; from half of the lanes on, 12.2,
-    // 1.41 and 9.65 with 16 steps).
+    // While three of the launch's lanes in four wait, they are half as long:
+    // issue slots are free and what counts is how fast work spreads.  Against
+    // other rules on the same inputs, the other rule first, in ms:
+    //   never in the device loop: one random 15-puzzle 1.54 and 1.46, 50
+    //     24-puzzles 7.77 and 7.51, 100 Manhattan walks 8.78 and 8.80;
+    //   that, and in rounds from 9 lanes in 16 on: 1.03 and 0.94, 11.84 and
+    //     11.59, 9.22 and 9.26;
+    //   from half of the lanes on: 1.77 and 1.78, 9.18 and 9.29, 7.97 and 7.80.
     int steps = MULTI ? P.steps : P.steps + P.steps / 4;
     if ((int32_t)(hd - tl) > (int32_t)(48u * P.spread)) steps = (P.steps + 1) / 2;
     for (int s = 0; s < steps; ++s) {
@@ -1448,9 +1451,12 @@ cudaError_t launch_split_level(int w, bool pdb, int num_sms, const SplitArgs &A,
 }
 
 // Host launchers (template kernels stay in this translation unit).
+struct SearchShape {
+  void (*kern)(RoundParams) = nullptr;
+  int grid = 0, block = 0;
+};
 template <bool MULTI>
-static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, int num_sms, const RoundParams &P,
-                               cudaStream_t st, int *lanes_out) {
+static cudaError_t search_shape(int w, bool pdb, int block, int blocks_per_sm, int num_sms, SearchShape *out) {
   void (*kern)(RoundParams) = nullptr;
 #define SP_PICK(W, PD, B, WD) \
   if (w == W && pdb == PD && block == B) kern = search_round_kernel<W, PD, B, WD, MULTI>;
@@ -1475,21 +1481,31 @@ static cudaError_t launch_impl(int w, bool pdb, int block, int blocks_per_sm, in
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
   }
-  const int grid = num_sms * per_sm;
-  if (lanes_out) *lanes_out = grid * block;
-  kern<<<grid, block, 0, st>>>(P);
+  *out = SearchShape{kern, num_sms * per_sm, block};
+  return cudaSuccess;
+}
+
+static cudaError_t search_shape(int w, bool pdb, int block, int blocks_per_sm, int num_sms, bool multi,
+                                SearchShape *out) {
+  return multi ? search_shape<true>(w, pdb, block, blocks_per_sm, num_sms, out)
+               : search_shape<false>(w, pdb, block, blocks_per_sm, num_sms, out);
+}
+
+cudaError_t search_lanes(int w, bool pdb, int block, int blocks_per_sm, int num_sms, bool multi, uint32_t *lanes) {
+  SearchShape x;
+  const cudaError_t e = search_shape(w, pdb, block, blocks_per_sm, num_sms, multi, &x);
+  if (e == cudaSuccess) *lanes = (uint32_t)(x.grid * x.block);
+  return e;
+}
+
+cudaError_t launch_search(int w, bool pdb, int block, int blocks_per_sm, int num_sms, bool multi, const RoundParams &P,
+                          cudaStream_t st) {
+  SearchShape x;
+  const cudaError_t e = search_shape(w, pdb, block, blocks_per_sm, num_sms, multi, &x);
+  if (e != cudaSuccess) return e;
+  x.kern<<<x.grid, x.block, 0, st>>>(P);
   note_launch();
   return cudaGetLastError();
-}
-
-cudaError_t launch_search_round(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *lanes_out) {
-  return launch_impl<false>(w, pdb, block, blocks_per_sm, num_sms, P, st, lanes_out);
-}
-
-cudaError_t launch_search_multi(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *lanes_out) {
-  return launch_impl<true>(w, pdb, block, blocks_per_sm, num_sms, P, st, lanes_out);
 }
 
 cudaError_t launch_pool_init(Task *tasks, const uint32_t *n_emit, const uint32_t *direct, uint32_t n_direct,

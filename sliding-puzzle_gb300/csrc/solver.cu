@@ -245,7 +245,6 @@ struct sp_solver {
   uint8_t *d_pdb = nullptr;
   bool pdb_ready = false;
   uint32_t import_mask = 0;
-  int last_lanes = 0;       // lanes of the last search launch
   uint32_t last_emitted = 0;
   // split pre-pass buffers
   uint32_t *d_cnt = nullptr;  // [level a, level b, emitted, error]
@@ -697,6 +696,15 @@ int ensure_pool(sp_solver *s, size_t n_init) {
   return SP_OK;
 }
 
+// Lanes of a round's launch or, with `multi`, of the device loop's: the two
+// kernels differ, and what depends on their lanes must not hang on which of
+// them ran last.
+int lanes_of(sp_solver *s, bool multi, uint32_t *lanes) {
+  const int block = s->cfg.threads_per_block == 128 ? 128 : 256;
+  SP_CUDA(s, search_lanes(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, multi, lanes));
+  return SP_OK;
+}
+
 // Limits and solution records for n instances, two of each per instance: the
 // device loop keeps one per iteration parity.
 int ensure_instances(sp_solver *s, size_t n) {
@@ -821,11 +829,11 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
   P.timeout_ns = (unsigned long long)s->cfg.timeout_ms * 1000000ull;
   P.poll_ns = SP_POLL_NS;
   const int block = s->cfg.threads_per_block == 128 ? 128 : 256;
-  const uint32_t lanes = (uint32_t)(s->last_lanes > 0 ? s->last_lanes : s->num_sms * 1024);
+  uint32_t lanes = 0;
+  if ((rc = lanes_of(s, multi, &lanes))) return rc;
   P.reserve = s->cfg.donate_reserve < 0 ? 0u : s->cfg.donate_reserve > 0 ? (uint32_t)s->cfg.donate_reserve
                                                                           : lanes / 16u;
   P.spread = std::max(1u, lanes / 64u);  // lanes / 32 and / 16: 100 random 15-puzzles 1.4 and 2.5 % slower
-  int n_lanes = 0;
   if (multi) {
     MultiBufs &m = s->mb;
     P.inst_iter = m.iter;
@@ -851,12 +859,8 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
     P.static_split = (s->cfg.lb_mode == SP_LB_STATIC_STEAL || s->cfg.lb_mode == SP_LB_LEARNED) ? 1 : 0;
     P.handback_nodes = (unsigned long long)s->cfg.handback_nodes;
     P.sub_growth = m.use_growth ? m.growth : nullptr;
-    SP_CUDA(s, launch_search_multi(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, P,
-                                   s->st, &n_lanes));
-  } else {
-    SP_CUDA(s, launch_search_round(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, P,
-                                   s->st, &n_lanes));
   }
+  SP_CUDA(s, launch_search(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, multi, P, s->st));
   SP_CUDA(s, cudaEventRecord(s->ev1, s->st));
   SP_CUDA(s, s->h_ctl.reserve(1));
   SP_CUDA(s, s->h_sub_nodes.reserve(std::max<size_t>(n_subs, 1)));
@@ -874,7 +878,6 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
   SP_CUDA(s, cudaEventElapsedTime(ms, s->ev0, s->ev1));
   s->stats.d2h_bytes += sizeof(PoolCtl) + 16 + n_subs * 8 + n_sol * sizeof(Solution);
   s->stats.kernel_launches += 2;
-  s->last_lanes = n_lanes;
   s->last_emitted = s->h_cnt.p[2];
   if (!s->h_ctl.p->error && s->h_cnt.p[3]) s->h_ctl.p->error = (int32_t)s->h_cnt.p[3];
   return SP_OK;
@@ -988,8 +991,9 @@ int plan_round(sp_solver *s, std::vector<Instance> &inst, const std::vector<int3
       }
     }
   }
-  const double lanes = s->last_lanes > 0 ? (double)s->last_lanes : (double)s->num_sms * 1024.0;
-  const double T = total / (lanes * (double)SP_SPLIT_PIECES_PER_LANE);
+  uint32_t lanes = 0;
+  if (const int rc = lanes_of(s, false, &lanes)) return rc;
+  const double T = total / ((double)lanes * (double)SP_SPLIT_PIECES_PER_LANE);
   static const size_t pow3[12] = {1, 3, 9, 27, 81, 243, 729, 2187, 6561, 19683, 59049, 177147};
   auto bound = [&](int kk) { return kk ? 4 * pow3[kk - 1] : (size_t)0; };
   const int kcap = std::min(10, std::max(1, s->cfg.static_split_cap));
@@ -1410,16 +1414,17 @@ int solve_impl(sp_solver *s, const uint8_t *tiles, int nin, sp_result *res) {
   // root set: uniform-depth tree expansion to >= frontier_target leaves per
   // instance, on the device
   auto t_front = std::chrono::steady_clock::now();
-  // a batch's root set is capped near 8 roots per resident lane: more roots
+  // a batch's root set is capped near 8 roots per lane of a round: more roots
   // than that add work and no balance (donation splits what is left)
   size_t live = 0;
   for (auto &I : inst) live += !I.done;
-  const double lanes = s->last_lanes > 0 ? (double)s->last_lanes : (double)s->num_sms * 768.0;
-  int target = std::max(1, s->cfg.frontier_target);
-  if (live) target = std::min(target, std::max(32, (int)(8.0 * lanes / (double)live)));
-  size_t n_subs = 0;
-  int rc = build_root_sets(s, tiles, inst, target, &n_subs);
+  uint32_t lanes = 0;
+  int rc = lanes_of(s, false, &lanes);
   if (rc) return rc;
+  int target = std::max(1, s->cfg.frontier_target);
+  if (live) target = std::min(target, std::max(32, (int)(8.0 * (double)lanes / (double)live)));
+  size_t n_subs = 0;
+  if ((rc = build_root_sets(s, tiles, inst, target, &n_subs))) return rc;
   if ((rc = ensure_instances(s, inst.size()))) return rc;
   SP_CUDA(s, s->h_limits.reserve(inst.size()));
   s->stats.frontier_ms += ms_since(t_front);
@@ -1850,10 +1855,8 @@ int sp_selftest_stall(sp_solver *s, int timeout_ms, int32_t *device_status) {
   P.poll_ns = SP_POLL_NS;
   P.reserve = 0;
   P.spread = 1;
-  int n_lanes = 0;
   const int block = s->cfg.threads_per_block == 128 ? 128 : 256;
-  SP_CUDA(s, launch_search_round(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, P, s->st,
-                                 &n_lanes));
+  SP_CUDA(s, launch_search(s->w, s->heur == SP_HEUR_PDB, block, s->cfg.blocks_per_sm, s->num_sms, false, P, s->st));
   SP_CUDA(s, s->h_ctl.reserve(1));
   SP_CUDA(s, cudaMemcpyAsync(s->h_ctl.p, s->d_ctl, sizeof(PoolCtl), cudaMemcpyDeviceToHost, s->st));
   SP_CUDA(s, cudaStreamSynchronize(s->st));

@@ -63,12 +63,14 @@ struct RoundParams {
 };
 constexpr int kGrowthSlacks = 8;
 
-// One threshold round: grid = num_sms * blocks_per_sm (0 = occupancy maximum).
-cudaError_t launch_search_round(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *lanes_out);
-// The whole threshold loop of a batch in one launch (multi-iteration mode).
-cudaError_t launch_search_multi(int w, bool pdb, int block, int blocks_per_sm, int num_sms,
-                                const RoundParams &P, cudaStream_t st, int *lanes_out);
+// One threshold round or, with `multi`, the whole threshold loop of a batch in
+// one launch (multi-iteration mode).  Blocks of `block` threads, blocks_per_sm
+// of them on each SM; 0: the occupancy maximum or, for a round in blocks of 256,
+// one block of 1024 (24-puzzle PDB 768) threads per SM (search.cu).
+cudaError_t launch_search(int w, bool pdb, int block, int blocks_per_sm, int num_sms, bool multi, const RoundParams &P,
+                          cudaStream_t st);
+// The lanes of that launch.
+cudaError_t search_lanes(int w, bool pdb, int block, int blocks_per_sm, int num_sms, bool multi, uint32_t *lanes);
 // Publish the round's tasks and reset the pool control block: the split
 // pieces (*n_emit of them, 0 when null), which the pre-pass has written to the
 // ring's first slots, then the direct tasks.
