@@ -789,7 +789,8 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
       return false;
     }
     const uint32_t *path = P.tasks[s].path;
-    for (int wi = 0; 16 * wi < plen; ++wi) prefix[wi] = __ldcg(path + wi);
+    const int moves = min(plen, kMaxPath);  // a record with more is refused below
+    for (int wi = 0; 16 * wi < moves; ++wi) prefix[wi] = __ldcg(path + wi);
     st_release(&P.seq[s], slot + P.cap);  // the copies above complete before the slot is reused
     splitk = flags & 0x3Fu;
     const uint32_t parity = flags >> 6 & 1u;
@@ -813,7 +814,8 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     }
     blank = (int)((b1.z >> 8) & 0xFFu);
     if (!mask) return false;  // a null task
-    if (blank >= N) {         // corrupt record: never index off the board
+    const uint32_t word[7] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z};
+    if (!record_ok(W, word, plen)) {  // corrupt: never index out of range
       set_error(SP_ERR_ARG, 0x100u);
       return false;
     }
@@ -952,13 +954,14 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
       k = gen ? lev + 1 : lev;
       if (gen && (nh == 0 || lev >= krare)) {
         if (R::kDeep > 0 && lev >= R::kShared) deep[lev - R::kShared] = up | oldr << 8 | oldf << 16;
-        if (nh == 0) record_goal();
+        const bool full = lev >= min(R::kMaxLev - 1, kMaxPath - plen);  // no room for a path that long
+        if (nh == 0 && !full) record_goal();
         // split task with `splitk` levels left: this child (already counted
         // as generated) becomes a task of its own with one level fewer
         // (published outside the step loop), so a heavy root is split
         // breadth-first by many lanes; the lane then steps back
         if (splitk && lev == 0) ev = kStepEmit;
-        if (lev >= min(R::kMaxLev - 1, kMaxPath - plen)) {
+        if (full) {
           set_error(SP_ERR_STACK_OVERFLOW, (uint32_t)(plen + lev));
           ev = kStepDone;
         }

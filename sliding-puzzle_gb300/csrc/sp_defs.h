@@ -112,6 +112,22 @@ struct alignas(16) Task {
   uint32_t pad;
 };
 static_assert(sizeof(Task) == 80, "Task layout");
+// Whether a record can be used without an index leaving a table, the board or
+// the path: the blank on the board, every tile byte below w * w, plen moves in
+// the path.  `word`: the record's first seven words (board, blank); a bad one
+// is reported instead of searched.
+SP_HD bool record_ok(int w, const uint32_t (&word)[7], int plen) {
+  uint32_t bad = 0;  // bit 7 of a byte: its tile is too large
+  if (w == 4) {
+    bad = (word[0] | word[1] | word[2] | word[3]) & 0xF0F0F0F0u;
+  } else {
+    for (int q = 0; q < 7; ++q) {
+      const uint32_t x = q < 6 ? word[q] : word[q] & 0xFFu;
+      bad |= (((x & 0x7F7F7F7Fu) + 0x67676767u) | x) & 0x80808080u;  // 25 + 0x67 = 0x80
+    }
+  }
+  return !bad && (int)((word[6] >> 8) & 0xFFu) < w * w && plen <= kMaxPath;
+}
 constexpr int kMaxBudget = 30000;  // no sum of table bytes and moves comes near
 
 // One goal per instance: moves below its SubRoot.  `best` is
