@@ -32,7 +32,8 @@
 // distance as the reference's init_mdist / init_movable_table do,
 // src_horie/idas_parallel_host.c:88-129).  With a table whose reverse moves
 // do not take back what the moves added, h depends on the whole walk so far
-// and one thread walks the root alone.  Allocates nothing; launches on the
+// and one thread walks the root alone; so do the board and h of a root without
+// a blank, which leaves its block's roots to one thread each too.  Allocates nothing; launches on the
 // caller's stream and returns, like the reference.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(T) first_path_kernel(const uint8_t *input, int
       if (!t) r.blank = c;
       else r.h += abs(c / kW - (int)t / kW) + abs(c % kW - (int)t % kW);
     }
+    if (r.tile_at(r.blank)) s_alone = 1;
     s_board[tid] = r.b;
     s_blank[tid] = (uint8_t)r.blank;
     s_h[tid] = (uint8_t)r.h;
