@@ -704,7 +704,8 @@ def main():
                 traffic = float(line.split(":")[1])
     roofline = _sector_roofline(nodes, kms, peaks["l2_random_reads_per_s"], "l2-random", slide.pdb_table_bytes(4))
     roofline.update({
-        "traffic": traffic, "kernel": "search_round_kernel<4,pdb> (+ split pre-pass and pool set-up)",
+        "traffic": traffic, "kernel": "search_round_kernel<4,pdb> (device loop), search_sm_kernel<4,pdb> (rounds) "
+                                      "(+ split pre-pass and pool set-up)",
         "int_issue": _int_roofline(nodes, kms, peaks["int_ops_per_s"]),
         "hbm_copy": {"peak": hbm_peak, "peak_kind": hbm_kind, "unit": "GB/s",
                      "frac_if_every_lookup_went_to_dram": nodes * BYTES_PER_NODE / (kms / 1000.0) / 1e9 / hbm_peak,

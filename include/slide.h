@@ -75,8 +75,12 @@ typedef struct {
                                 reference's BLOCK_NUM is 2048);
                                 a batch is capped near 8 per lane of a round
                                 (at least 32 per instance) */
-  int32_t threads_per_block; /* 128 or 256 */
-  int32_t blocks_per_sm;     /* 0 = occupancy maximum */
+  int32_t threads_per_block; /* 128 or 256 (default) */
+  int32_t blocks_per_sm;     /* 0 = occupancy maximum, but with 256 threads a threshold
+                                round runs in one block per SM, of 1024 threads (24-puzzle
+                                with tables: 768); a number gives it that many blocks of
+                                256 (the occupancy maximum is 4 for 15-puzzle rounds with
+                                tables, else 3) */
   int32_t lb_mode;           /* sp_lb_mode */
   int32_t donate_min_slack;  /* donate a branch only if limit - depth >= this */
   int32_t steps_per_poll;    /* DFS steps between task-pool polls */
@@ -230,8 +234,9 @@ int sp_dfs_round_md_noalloc(int width, const uint8_t *d_roots, const int32_t *d_
  * left, down without undoing the last one, and stops at its first goal.
  * Row i of d_plan (device memory, n*SP_PLAN_STRIDE bytes) receives
  * [len, move_1 ... move_len] or [-1] when the root has no goal within the
- * limit ([-2]: the root's search ran past 30 s, which only a table that lets
- * h fall without bound can cause).  d_h_diff_table (16*16*4 signed bytes,
+ * limit ([-2]: the root's search ran past 30 s, which takes a table that lets
+ * h fall without bound or a tree as large; the up to 128 roots that share a
+ * block's threads start together).  d_h_diff_table (16*16*4 signed bytes,
  * [tile][its cell][blank's move], the reference's init_mdist layout) and
  * d_movable_table (16*4 bytes, [cell][move]; a move off the board is never
  * made, whatever the table says) are device tables as the

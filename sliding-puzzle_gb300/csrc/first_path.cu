@@ -13,7 +13,9 @@
 // or [-1].  The root's own depth is not counted: roots are searched as if at
 // depth 0.  No node counts: the reference reports none on this path.  Two
 // guards the reference lacks: a path never grows past the plan row (251
-// moves), and a root searched for more than 30 s gives up with [-2].
+// moves), and a root that 30 s of its block's search have not settled gives up
+// with [-2] (a block's roots start together and share its threads; a root never
+// has fewer than one while it is open).
 //
 // GPU shape: a block for one root, or for several when there are many.  A
 // depth-first search visits its tree's nodes in the order of their move

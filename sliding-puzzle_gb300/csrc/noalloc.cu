@@ -42,8 +42,14 @@ namespace {
 constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
-constexpr uint32_t kNoAllocPoolCap = 1u << 17;  // ring slots (power of two)
+// Ring slots (a power of two).  Fewer than a round's lanes (1024 per SM, 155648
+// on 152 SMs), all of which may hold a claim: a claim takes no slot, and of two
+// lanes whose claims fall on one slot its sequence number says whose turn it
+// is.  A slot is taken from publication to claim, and lanes give work away
+// only while fewer than P.reserve (a 16th of the lanes) tasks are unclaimed.
+constexpr uint32_t kNoAllocPoolCap = 1u << 17;
 constexpr int kNoAllocMaxRoots = 16384;
+static_assert((uint32_t)kNoAllocMaxRoots <= kNoAllocPoolCap / 2, "the roots leave half of the ring to donations");
 constexpr int kMaxDevices = 64;
 
 // layout of the scratch array

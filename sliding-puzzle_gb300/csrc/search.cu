@@ -31,7 +31,8 @@
 //    and 5-9): 100 random 15-puzzles 28.8 -> 19.7 -> 15.9 ms, 4096 mixed ones
 //    348 -> 211 -> 156 ms (the large rounds 70 -> 116 -> 140 G nodes/s), 100
 //    Manhattan walks 29.2 -> 18.9 -> 8.9 ms, 16384 24-puzzle roots 166 -> 101
-//    -> 59 ms;
+//    -> 59 ms (each chain on inputs of its own: other instances of a kind take up
+//    to a fifth more or less);
 //  * load balance by a device task pool: lanes claim slots warp-aggregated
 //    (ballot + one atomicAdd per warp); claims may run ahead of the pool's
 //    tail, and while any lane waits, busy lanes donate the untried moves of
@@ -393,17 +394,18 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
   }
 }
 
-// Most lanes of a warp that donate in one pass of its loop (4 / 8 / 16: one
-// random 15-puzzle 2.87 / 2.64 / 2.57 ms, 100 of them 19.2 / 18.8 / 18.9).
+// Most lanes of a warp that donate in one pass of its loop (8 / 16 / 32: one
+// random 15-puzzle 1.87 / 1.81 / 1.81 ms, 100 of them 17.84 / 17.71 / 17.76, a
+// walk of 40 moves 0.78 / 0.75 / 0.75).
 #ifndef SP_MAX_DONORS
 #define SP_MAX_DONORS 16
 #endif
 
 // Longest sleep of a warp with no lane searching between pool polls (ns): a
-// new iteration waits for it, other warps lose issue slots to the polls (512 /
-// 2048 / 4096 / 16384: one random 15-puzzle 3.4 / 2.8 / 2.65 / 2.76 ms, 50
-// 24-puzzles 19.8 / 19.2 / 19.2 / 20.0, a walk of 40 moves 0.89 / 0.72 / 0.70 /
-// 0.84).
+// new iteration waits for it, other warps lose issue slots to the polls (2048 /
+// 4096 / 16384: one random 15-puzzle 1.93 / 1.81 / 2.12 ms, 100 of them 17.90 /
+// 17.72 / 18.75, 50 24-puzzles 45.2 / 45.1 / 45.9, a walk of 40 moves 0.75 / 0.75
+// / 0.97).
 #ifndef SP_MAX_BACKOFF_NS
 #define SP_MAX_BACKOFF_NS 4096
 #endif
@@ -421,8 +423,8 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
 // 68.2).  Threads, 15-puzzle: 768 / 896 / 1024 166 / 157 / 156 ms;
 // 24-puzzle, whose rows are longer, so that more threads leave it fewer shared
 // levels: 640 / 768 / 896 / 1024 65.3 / 63.8 / 70.3 / 72.7.
-// Blocks of 128 and 256 threads stay for a caller that asks for them or for a
-// number of blocks per SM.  Manhattan reads no tables and is bound by issue and
+// Blocks of 128 threads, and of 256 in a named number per SM, stay for a caller
+// that asks for them.  Manhattan reads no tables and is bound by issue and
 // shared memory's latency: 1024 threads (blocks of 256, 768 an SM / one of 768
 // / 896 / 1024: 2048 24-puzzle roots 11.25 / 11.08 / 10.31 / 10.00 ms, 100
 // 15-puzzle walks 9.47 / 9.35 / 9.03 / 9.10).

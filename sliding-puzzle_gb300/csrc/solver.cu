@@ -675,8 +675,9 @@ bool replay_ok(int w, const uint8_t *tiles, const uint8_t *moves, int len) {
   return true;
 }
 
-// Ring capacity: a power of two holding the round's root tasks plus room for
-// a waiting claim from every resident lane.
+// Ring capacity: a power of two holding the round's root tasks and pieces, and
+// as many donations and claims besides as lanes can be resident (80 bytes a
+// slot: 160 MB for a batch, whose device loop may split into 2^20 pieces).
 int ensure_pool(sp_solver *s, size_t n_init) {
   size_t need = (size_t)1 << 20;
   while (need < n_init + ((size_t)1 << 19)) need <<= 1;
