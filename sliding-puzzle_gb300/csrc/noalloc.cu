@@ -46,7 +46,7 @@ constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign;
 // on 152 SMs), all of which may hold a claim: a claim takes no slot, and of two
 // lanes whose claims fall on one slot its sequence number says whose turn it
 // is.  A slot is taken from publication to claim, and lanes give work away
-// only while fewer than P.reserve (a 16th of the lanes) tasks are unclaimed.
+// only while fewer than P.reserve (48 per SM) tasks are unclaimed.
 constexpr uint32_t kNoAllocPoolCap = 1u << 17;
 constexpr int kNoAllocMaxRoots = 16384;
 static_assert((uint32_t)kNoAllocMaxRoots <= kNoAllocPoolCap / 2, "the roots leave half of the ring to donations");
@@ -251,6 +251,7 @@ extern "C" int sp_dfs_round_md_noalloc(int width, const uint8_t *d_roots, const 
     P.poll_ns = 4000;
     uint32_t lanes = 0;
     if (search_lanes(width, false, 256, 0, num_sms, false, &lanes) != cudaSuccess) return SP_ERR_CUDA;
+    lanes = donation_lanes(lanes, num_sms);
     P.reserve = lanes / 16u;
     P.spread = lanes / 64u;
     if (launch_search(width, false, 256, 0, num_sms, false, P, st) != cudaSuccess) return SP_ERR_CUDA;

@@ -1131,14 +1131,16 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     // next iteration waits for the last one's tasks (32 / 40 / 48 steps: 100
     // random 15-puzzles 17.4 / 16.9 / 16.9 ms, 2048 24-puzzle roots 11.8 / 11.3
     // / 11.2, 50 24-puzzles 12.7 / 12.9 / 12.9).
-    // While three of the launch's lanes in four wait, they are half as long:
-    // issue slots are free and what counts is how fast work spreads.  Against
-    // other rules on the same inputs, the other rule first, in ms:
+    // While as many lanes wait as are three quarters of 768 per SM (of a
+    // round's 1024, 9 in 16), they are half as long: issue slots are free and
+    // what counts is how fast work spreads.  Against other rules on the same
+    // inputs, the other rule first, in ms:
     //   never in the device loop: one random 15-puzzle 1.54 and 1.46, 50
     //     24-puzzles 7.77 and 7.51, 100 Manhattan walks 8.78 and 8.80;
-    //   that, and in rounds from 9 lanes in 16 on: 1.03 and 0.94, 11.84 and
-    //     11.59, 9.22 and 9.26;
-    //   from half of the lanes on: 1.77 and 1.78, 9.18 and 9.29, 7.97 and 7.80.
+    //   in rounds of 1024 from three lanes in four on: one random 15-puzzle
+    //     1.84 and 1.83, 100 of them 11.93 and 11.87, 4096 mixed ones 174.7 and
+    //     174.1;
+    //   from half of all lanes on: 24-puzzles 9.18 and 9.29, walks 7.97 and 7.80.
     int steps = MULTI ? P.steps : P.steps + P.steps / 4;
     if ((int32_t)(hd - tl) > (int32_t)(48u * P.spread)) steps = (P.steps + 1) / 2;
     for (int s = 0; s < steps; ++s) {

@@ -832,9 +832,10 @@ int launch_round(sp_solver *s, const RoundPlan &plan, size_t n_subs, size_t n_in
   const int block = s->cfg.threads_per_block == 128 ? 128 : 256;
   uint32_t lanes = 0;
   if ((rc = lanes_of(s, multi, &lanes))) return rc;
+  const uint32_t givers = donation_lanes(lanes, s->num_sms);
   P.reserve = s->cfg.donate_reserve < 0 ? 0u : s->cfg.donate_reserve > 0 ? (uint32_t)s->cfg.donate_reserve
-                                                                          : lanes / 16u;
-  P.spread = std::max(1u, lanes / 64u);  // lanes / 32 and / 16: 100 random 15-puzzles 1.4 and 2.5 % slower
+                                                                          : givers / 16u;
+  P.spread = std::max(1u, givers / 64u);  // lanes / 32 and / 16: 100 random 15-puzzles 1.4 and 2.5 % slower
   if (multi) {
     MultiBufs &m = s->mb;
     P.inst_iter = m.iter;

@@ -26,7 +26,7 @@ struct RoundParams {
   int32_t steps;
   int32_t donate;
   uint32_t reserve;   // donate while fewer than this many tasks are queued
-  uint32_t spread;    // a 64th of the lanes: one extra donor per warp per `spread` missing tasks
+  uint32_t spread;    // a 64th of donation_lanes: one extra donor per warp per `spread` missing tasks
   uint32_t pad1;
   unsigned long long timeout_ns;
   unsigned long long poll_ns;  // min interval of a block's global pool poll
@@ -71,6 +71,15 @@ cudaError_t launch_search(int w, bool pdb, int block, int blocks_per_sm, int num
                           cudaStream_t st);
 // The lanes of that launch.
 cudaError_t search_lanes(int w, bool pdb, int block, int blocks_per_sm, int num_sms, bool multi, uint32_t *lanes);
+// The lanes that a launch's donation reserve (a 16th) and donors per pass (a
+// 64th to one more donor) go by: its own, 768 per SM at most.  With all 1024
+// of a round, 2048 24-puzzle roots by Manhattan take 7.93 ms instead of 7.84,
+// 100 random 15-puzzles 11.98 instead of 11.87, 4096 mixed ones 175.4 instead
+// of 174.1.
+inline uint32_t donation_lanes(uint32_t lanes, int num_sms) {
+  const uint32_t most = (uint32_t)num_sms * 768u;
+  return lanes < most ? lanes : most;
+}
 // Publish the round's tasks and reset the pool control block: the split
 // pieces (*n_emit of them, 0 when null), which the pre-pass has written to the
 // ring's first slots, then the direct tasks.
