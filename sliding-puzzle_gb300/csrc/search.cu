@@ -383,6 +383,7 @@ __device__ __noinline__ void warp_advance(const RoundParams &P, uint32_t i, uint
       t0 = atomicAdd(&ctl->tail, nb + nb2);
     }
     t0 = __shfl_sync(FULL, t0, 0);
+    __syncwarp();  // orders lane 0's counts before the other lanes' publications, which the shuffle does not
     for (uint32_t b = lane; b < nb + nb2; b += 32) {
       const bool second = b >= nb;
       const uint32_t q0 = (second ? b - nb : b) * kBulk, left = (second ? na2 : na) - q0;
