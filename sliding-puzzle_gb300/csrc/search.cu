@@ -1001,6 +1001,11 @@ __device__ __forceinline__ void search_round(const RoundParams &P) {
     if (MULTI) {
       unsigned pend = __ballot_sync(FULL, events & kAdvance);
       while (pend) {
+        // all lanes read the instance in s_cold0 and the loads and goals of the
+        // tasks whose end the marked lane has seen, and write the s_hist that
+        // the advance before used
+        __threadfence();
+        __syncwarp();
         const int src = __ffs(pend) - 1;
         pend &= pend - 1u;
         warp_advance(P, s_cold0[(tid & ~31) + src], s_hist[tid >> 5]);

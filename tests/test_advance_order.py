@@ -18,3 +18,13 @@ def test_a_warp_barrier_follows_the_count_of_an_iterations_tasks():
     count = src.index("atomicAdd(&ctl->outstanding, na + na2)")
     between = src[count:src.index("publish_root(P, t0 + b", count)]
     assert re.search(r"__shfl_sync\([^;]*;\s*__syncwarp\(\);\s*for \(", between), between
+
+
+def test_a_warp_waits_before_it_reads_the_instances_to_advance():
+    """A lane leaves the instance it has finished an iteration of in shared
+    memory, and all lanes of its warp read it: a vote is no barrier for memory,
+    so a fence and a warp barrier come before each advance."""
+    src = _source()
+    vote = src.index("while (pend)", src.index("__ballot_sync(FULL, events & kAdvance)"))
+    between = src[vote:src.index("warp_advance(P, s_cold0", vote)]
+    assert re.search(r"\{\s*__threadfence\(\);\s*__syncwarp\(\);", between), between
